@@ -230,7 +230,8 @@ qas_status qas_bc_map(const qas_grid *grid, const qas_bc *bc, int group, int fie
 /* Diagnostics: per-kernel device time measured live with CUDA events on the context's
  * stream.  Runs `nsteps` exec_ steps (the same work as qas_run, launched eagerly) with an
  * event pair around every kernel launch and returns, per kernel, the number of launches and
- * the summed durations.  *count receives the number of entries written (<= max_entries). */
+ * the summed durations (in 2D with the face sweeps in their two-kernel form unless
+ * QAS_OPT_FUSED_SWEEP was set, so that the reconstruction and the flux are timed apart).  *count receives the number of entries written (<= max_entries). */
 typedef struct {
   char name[32];
   long long launches;
@@ -266,9 +267,10 @@ qas_status qas_set_gravity(qas_ctx *ctx, const double *phi_g);
 
 /* Tuning options (defaults are the measured best on B200).
  *   QAS_OPT_FUSED_SWEEP: 0 = reconstruction and Riemann flux of each direction in two
- *   kernels with the face states in HBM (default in 1D and 2D); 1 = one fused sweep kernel
- *   per direction, the face states kept on chip (default in 3D; 4th-order interpolation only,
- *   other orders keep the two kernels).
+ *   kernels with the face states in HBM (default in 1D); 1 = one fused sweep kernel per
+ *   direction, the face states kept on chip (default in 3D; 4th-order interpolation only,
+ *   other orders keep the two kernels).  The 2D default fuses x, and y for the HLLD solvers and
+ *   on small grids.
  *   QAS_OPT_LR_STAGING: 1 = the reconstruction stages its stencils in shared memory with
  *   TMA tensor copies (available for 2D/3D, 4th-order interpolation, even padded x extent;
  *   QAS_ERR_UNSUPPORTED otherwise); 0 = it reads them from global memory (default: measured

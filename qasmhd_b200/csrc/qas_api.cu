@@ -116,9 +116,10 @@ struct qas_ctx {
   qas_status latched = QAS_OK;
   // thread-block tile (x,y,z extents, 128 threads) of every cell kernel, by kernel id
   dim3 tile[32];
-  // face sweep form: two kernels with the face states in HBM, or one fused kernel (the
-  // default in 3D, set at creation)
-  bool fused = false;
+  // face sweep form per axis (bit a): one fused kernel, else two kernels with the face states in
+  // HBM; chosen at creation (fused_axes), or for every axis by QAS_OPT_FUSED_SWEEP (fused_set)
+  unsigned fused = 0;
+  bool fused_set = false;
   int sweep_seg[3] = {0, 0, 0};  // segment length of the fused y / z sweeps (0: not chosen yet)
   // live per-kernel timing (qas_profile_run): an event pair around every launch
   bool prof = false;
@@ -506,27 +507,29 @@ void launch_flux(qas_ctx *c, int a)
   }
 }
 
-// segment length of the y / z sweeps: fewest cell computations per resident block slot over
-// the waves of blocks (each segment recomputes the cell before its first face)
+// faces per block of the y / z sweeps.  A block of four warps takes four cells a round, the cell
+// before its first face among them, so segments are 4k - 1 faces; the cost weighs the rounds of all
+// blocks (and a third of one for a block's start, its first loads) against the half block by which
+// the last ones finish late.  KH 128^3 (MLAU, z): 15 / 19 / 27 / 35 / 67 faces 328 / 332 / 329 /
+// 353 / 417 us.
 int sweep_seg(qas_ctx *c, int a, const void *fn)
 {
   if (c->sweep_seg[a] > 0) return c->sweep_seg[a];
   const Geo &g = c->geo;
   int dev = 0, sms = 148, occ = 1;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 128, 0) != cudaSuccess || occ < 1) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, SWB, 0) != cudaSuccess || occ < 1) {
     cudaGetLastError();
     occ = 1;
   }
-  const long long colb = ((long long)g.nx * (a == 1 ? g.nz : g.ny) + 127) / 128;
-  const long long slots = (long long)sms * occ;
+  const long long colb = ((long long)g.nx * (a == 1 ? g.nz : g.ny) + 31) / 32;
+  const double slots = (double)sms * occ;
   const int len = g.n[a] - 5;  // faces 3 .. n-3
   double best = 1e300;
-  int bseg = len;
-  for (int ns = 1; ns <= len; ns++) {
-    const int seg = (len + ns - 1) / ns;
-    const long long blocks = colb * ((len + seg - 1) / seg);
-    const double cost = (double)((blocks + slots - 1) / slots) * (seg + 1);
+  int bseg = 3;
+  for (int seg = 3; seg < len + 4; seg += 4) {
+    const double rounds = (seg + 1) / 4, blocks = (double)(colb * ((len + seg - 1) / seg));
+    const double cost = std::max(blocks / slots, 1.0) * (rounds + 0.35) + 0.5 * rounds;
     if (cost < best - 1e-9) {
       best = cost;
       bseg = seg;
@@ -536,25 +539,11 @@ int sweep_seg(qas_ctx *c, int a, const void *fn)
   return bseg;
 }
 
-// shared-memory carveout hint of the fused sweeps (percent of the SM's maximum; -1: the driver's
-// choice): the y / z sweeps read each stencil plane five times along their march, from L1
-// when the rest of the SM's 256 KB is left to it
-#ifndef QAS_SWEEP_CARVEOUT
-#define QAS_SWEEP_CARVEOUT -1
-#endif
 // choose the y / z segment lengths outside any stream capture (occupancy query); the fused
 // sweeps are built for 4th-order interpolation only (other orders take the two-kernel form)
 template <int RMN>
 void sweep_prepare_t(qas_ctx *c)
 {
-  if (QAS_SWEEP_CARVEOUT >= 0) {
-    const void *fns[6] = {(const void *)k_sweep_x<4, RMN, 0>, (const void *)k_sweep_m<4, RMN, 1, 0>,
-                          (const void *)k_sweep_m<4, RMN, 2, 0>, (const void *)k_sweep_x<4, RMN, -1>,
-                          (const void *)k_sweep_m<4, RMN, 1, -1>, (const void *)k_sweep_m<4, RMN, 2, -1>};
-    for (const void *f : fns)
-      cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, QAS_SWEEP_CARVEOUT);
-    cudaGetLastError();
-  }
   if (c->geo.dim >= 2) sweep_seg(c, 1, (const void *)k_sweep_m<4, RMN, 1, 0>);
   if (c->geo.dim >= 3) sweep_seg(c, 2, (const void *)k_sweep_m<4, RMN, 2, 0>);
 }
@@ -569,6 +558,18 @@ void sweep_prepare(qas_ctx *c)
   }
 }
 
+// the axes whose face states stay on chip by default (bit a).  3D: all.  2D: x, and y for the HLLD
+// solvers and on small grids, where a launch counts more than the march (OT / KH 1024^2, two kernels
+// against one, us: x HLLD 139 / 121, LHLLD 149 / 134, MLAU 152 / 139, Roe 162 / 162; y HLLD 138 / 136,
+// LHLLD 152 / 147, MLAU 147 / 157, Roe 161 / 178).  1D and the other orders: none.
+unsigned fused_axes(const qas_ctx *c)
+{
+  if (c->scheme.odr != 4 || c->geo.dim == 1) return 0u;
+  if (c->geo.dim == 3) return 7u;
+  const bool hlld = c->scheme.rmn == 1 || c->scheme.rmn == 2;
+  return hlld || c->geo.nd <= (1ll << 18) ? 3u : 1u;
+}
+
 template <int RMN, int PR>
 void launch_sweep_pr(qas_ctx *c, int a)
 {
@@ -577,18 +578,18 @@ void launch_sweep_pr(qas_ctx *c, int a)
     // warp w takes flattened cells [31w, 31w+32); the last cell needing a flux is total-1
     const long long total = (long long)(g.nx - 4) * g.ny * g.nz;
     const long long nwarps = (total - 2) / 31 + 1;
-    const unsigned nb = (unsigned)((nwarps + 3) / 4);
-    QL(c, KID_SWEEP, k_sweep_x<4, RMN, PR><<<nb, 128, 0, c->stream>>>(c->view, nwarps));
+    const unsigned nb = (unsigned)((nwarps + SWB / 32 - 1) / (SWB / 32));
+    QL(c, KID_SWEEP, k_sweep_x<4, RMN, PR><<<nb, SWB, 0, c->stream>>>(c->view, nwarps));
     return;
   }
-  const unsigned colb = (unsigned)(((long long)g.nx * (a == 1 ? g.nz : g.ny) + 127) / 128);
+  const unsigned colb = (unsigned)(((long long)g.nx * (a == 1 ? g.nz : g.ny) + 31) / 32);
   const int len = g.n[a] - 5;
   if (a == 1) {
     const int seg = sweep_seg(c, 1, (const void *)k_sweep_m<4, RMN, 1, 0>);
-    QL(c, KID_SWEEP, k_sweep_m<4, RMN, 1, PR><<<dim3(colb, (len + seg - 1) / seg), 128, 0, c->stream>>>(c->view, seg));
+    QL(c, KID_SWEEP, k_sweep_m<4, RMN, 1, PR><<<dim3(colb, (len + seg - 1) / seg), SWB, 0, c->stream>>>(c->view, seg));
   } else {
     const int seg = sweep_seg(c, 2, (const void *)k_sweep_m<4, RMN, 2, 0>);
-    QL(c, KID_SWEEP, k_sweep_m<4, RMN, 2, PR><<<dim3(colb, (len + seg - 1) / seg), 128, 0, c->stream>>>(c->view, seg));
+    QL(c, KID_SWEEP, k_sweep_m<4, RMN, 2, PR><<<dim3(colb, (len + seg - 1) / seg), SWB, 0, c->stream>>>(c->view, seg));
   }
 }
 template <int RMN>
@@ -652,7 +653,8 @@ long long stage_rest(qas_ctx *c, double c0, double c1)
   long long nk = 0;
   for (int a = 0; a < g.dim; a++) {
     if constexpr (ODR == 4) {
-      if (c->fused) {
+      // a profile run keeps the 2D stage's two kernels apart, to time each
+      if (((c->fused >> a) & 1) && !(c->prof && g.dim == 2 && !c->fused_set)) {
         switch (c->scheme.rmn) {
           case 0: launch_sweep<0>(c, a); break;
           case 1: launch_sweep<1>(c, a); break;
@@ -1001,6 +1003,7 @@ qas_status qas_create(qas_ctx **out, const qas_grid *grid, const qas_scheme *sch
   v.ctw = scheme->ctw ? 1 : 0;
   v.recon = scheme->char_mode;
   v.gam = gr.gam;
+  v.gm1i = 1.0 / (gr.gam - 1.0);
   v.dx = gr.dx;
   v.dy = gr.dim >= 2 ? gr.dy : 1.0;
   v.dz = gr.dim >= 3 ? gr.dz : 1.0;
@@ -1033,11 +1036,7 @@ qas_status qas_create(qas_ctx **out, const qas_grid *grid, const qas_scheme *sch
   // by FP64 dependency latency, and the staged form measured 9-35 % slower per launch
   c->lr_tma_ok = scheme->odr == 4 && setup_lr_tma(c);
   c->lr_tma = false;
-  // face sweep form: fused (face states never in HBM) in 3D, where it measured faster on B200
-  // (KH 256^3, MLAU: 2.78 ms per sweep against 1.90 + 1.21 ms for the two kernels, and a cooler
-  // step under the power cap); two kernels in 1D/2D, where the y sweep has too few columns to
-  // march long segments (OT 1024^2: 0.164 against 0.102 + 0.050 ms)
-  c->fused = g.dim == 3;
+  c->fused = fused_axes(c);
   if (c->fused) sweep_prepare(c);
   if (cudaMemsetAsync(c->d_dctl, 0, sizeof(DCtl), c->stream) != cudaSuccess) return fail(QAS_ERR_CUDA);
   if ((st = write_ctl(c)) != QAS_OK) return fail(st);
@@ -1641,13 +1640,14 @@ qas_status qas_set_option(qas_ctx *c, int option, int value)
   QAS_API_TRY
   if (!c) return QAS_ERR_INVALID;
   if (option == QAS_OPT_FUSED_SWEEP) {
-    const bool f = value != 0;
+    const unsigned f = value != 0 ? 7u : 0u;
     if (f != c->fused && c->graph) {  // the captured graph holds the other form
       cudaStreamSynchronize(c->stream);
       cudaGraphExecDestroy(c->graph);
       c->graph = nullptr;
     }
     c->fused = f;
+    c->fused_set = true;
     if (f) sweep_prepare(c);
     return QAS_OK;
   }
@@ -1660,6 +1660,8 @@ qas_status qas_set_option(qas_ctx *c, int option, int value)
       c->graph = nullptr;
     }
     c->lr_tma = t;
+    // the staged kernel is a reconstruction of its own: in 2D it takes the place of the fused axes too
+    if (c->geo.dim == 2 && !c->fused_set) c->fused = t ? 0u : fused_axes(c);
     return QAS_OK;
   }
   if (option == QAS_OPT_TEST_TMA_STALL) {

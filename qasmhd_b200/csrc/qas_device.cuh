@@ -11,13 +11,8 @@
 #pragma once
 
 #include <math.h>
+#include <string.h>
 
-#ifndef QAS_ZERO_INT
-#define QAS_ZERO_INT 0
-#endif
-#ifndef QAS_WCNS4_NOINLINE
-#define QAS_WCNS4_NOINLINE 0
-#endif
 #if defined(__CUDACC__)
 #include <cuda_runtime.h>
 #define QAS_HD __host__ __device__ __forceinline__
@@ -27,18 +22,70 @@
 
 namespace qas {
 
+
 // ---------------------------------------------------------------------------
 // common/common_func.h:4-31
 // ---------------------------------------------------------------------------
-// exact-zero test of the reconstruction's zero-preservation flags (x == 0.0, both signs); on
-// the device with QAS_ZERO_INT as an integer test of the bits, which keeps it off the FP64 pipe
-// (same truth value for every input, NaN included)
-QAS_HD bool is_zero(double x)
+QAS_HD bool is_zero(double x) { return x == 0.0; }
+
+// c*a + b for c a power of two: the product is exact, so the one rounding of the FMA is the
+// reference's (c*a overflowing or falling below the normal range aside, see wcns4_lr_fast)
+QAS_HD double p2fma(double c, double a, double b)
 {
-#if defined(__CUDA_ARCH__) && QAS_ZERO_INT
-  return (__double_as_longlong(x) << 1) == 0;
+#if defined(__CUDA_ARCH__)
+  return fma(c, a, b);
 #else
-  return x == 0.0;
+  return c * a + b;
+#endif
+}
+
+// high word of x, for range tests on the integer pipe
+QAS_HD unsigned hiword(double x)
+{
+#if defined(__CUDA_ARCH__)
+  return (unsigned)__double2hiint(x);
+#else
+  unsigned long long b;
+  memcpy(&b, &x, 8);
+  return (unsigned)(b >> 32);
+#endif
+}
+QAS_HD unsigned umax3(unsigned a, unsigned b, unsigned c)
+{
+  const unsigned t = a > b ? a : b;
+  return t > c ? t : c;
+}
+
+// 1/x rounded to nearest for normal x with 2^-1000 < |x| < 2^1000, without the general
+// division's range test and out-of-line path at every use: the hardware's approximation
+// (rcp.approx.ftz.f64), a third-order Newton step, then Markstein's correction (P. Markstein,
+// IBM J. Res. Dev. 34, 1990; Muller et al., Handbook of Floating-Point Arithmetic, division by
+// Newton-Raphson): a y within one ulp of 1/x gives the rounded reciprocal as y + y*(1 - x*y),
+// except for a significand of all ones, where it must come from above: the approximation's low
+// word (0) is set to 1, which leads there.  Compared with 1.0/x bit for bit in the GPU tests.
+QAS_HD double rcp_normal(double x)
+{
+#if defined(__CUDA_ARCH__)
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = __hiloint2double(__double2hiint(y), 1);
+  double e = fma(-x, y, 1.0);
+  e = fma(e, e, e);
+  y = fma(y, e, y);
+  e = fma(-x, y, 1.0);
+  return fma(y, e, y);
+#else
+  return 1.0 / x;
+#endif
+}
+
+// x with its sign flipped where neg (the reference's multiplication by +-1.0), on the integer pipe
+QAS_HD double flip(double x, bool neg)
+{
+#if defined(__CUDA_ARCH__)
+  return __hiloint2double(__double2hiint(x) ^ (neg ? (int)0x80000000 : 0), __double2loint(x));
+#else
+  return neg ? -x : x;
 #endif
 }
 
@@ -107,13 +154,7 @@ QAS_HD double lin_right(const double f[5])
 // 1st order, MUSCL minmod (common_interp.c:32-37), WCNS3 (:65-101),
 // WCNS4 (:102-150)
 // ---------------------------------------------------------------------------
-// QAS_WCNS4_NOINLINE: one out-of-line copy of the WCNS4 interpolation on the device instead of
-// one per characteristic field (smaller kernels, fewer instruction-cache misses)
-#if defined(__CUDACC__) && QAS_WCNS4_NOINLINE
-__host__ __device__ __noinline__ void wcns4_lr(const double f[5], double &fl, double &fr)
-#else
 QAS_HD void wcns4_lr(const double f[5], double &fl, double &fr)
-#endif
 {
   const double eps = 1e-40;
   double c1, c2;
@@ -150,6 +191,63 @@ QAS_HD void wcns4_lr(const double f[5], double &fl, double &fr)
   w1 *= dn;
   w2 = 1.0 - w0 - w1;
   fr = 0.125 * (+w2 * pr2 + w1 * pr1 + w0 * pr0);
+}
+
+// wcns4_lr with the same rounded results in fewer FP64 operations (115 -> 101 a field), the form the
+// kernels run:
+//  * a product by a power of two feeding a sum is one FMA (p2fma);
+//  * the candidates carry the final factor 1/8 in their coefficients (3/8 f instead of 3 f, ...;
+//    every intermediate is the reference's times an exact power of two), and 6 f, 3 f share
+//    one product;
+//  * the five reciprocals are rcp_normal: s^2 + 1e-40 is at least 1e-40, so only the upper
+//    end needs a test, left to the caller: hx receives the largest high word of the three
+//    denominators (of any NaN too, whose sign bit or exponent exceeds every finite value's), and
+//    the results hold for hx < WCNS_HX, 2^900.
+// Magnitudes below about 2^-1015, where a scaled intermediate leaves the normal range, are the
+// one place where the last bit may differ.
+constexpr unsigned WCNS_HX = 0x78300000u;
+QAS_HD void wcns4_lr_fast(const double f[5], double &fl, double &fr, unsigned &hx)
+{
+  const double eps = 1e-40;
+  const double g1 = 0.375 * f[1], g2 = 0.375 * f[2], g3 = 0.375 * f[3];
+  double c1, c2;
+  c1 = p2fma(8.0, g2, p2fma(-4.0, f[1], f[0]));
+  c2 = p2fma(-2.0, f[1], f[0]) + f[2];
+  double s0 = p2fma(0.25, c1 * c1, (13. / 12.) * c2 * c2);
+  c1 = f[1] - f[3];
+  c2 = p2fma(-2.0, f[2], f[1]) + f[3];
+  double s1 = p2fma(0.25, c1 * c1, (13. / 12.) * c2 * c2);
+  c1 = p2fma(8.0, g2, p2fma(-4.0, f[3], f[4]));
+  c2 = p2fma(-2.0, f[3], f[4]) + f[2];
+  double s2 = p2fma(0.25, c1 * c1, (13. / 12.) * c2 * c2);
+  s0 = s0 * s0 + eps;
+  s1 = s1 * s1 + eps;
+  s2 = s2 * s2 + eps;
+  hx = umax3(hiword(s0), hiword(s1), umax3(hx, hiword(s2), 0u));
+  s0 = rcp_normal(s0);
+  s1 = rcp_normal(s1);
+  s2 = rcp_normal(s2);
+  const double h2 = 1.875 * f[2];
+  const double pl0 = 0.375 * f[0] - 1.25 * f[1] + h2;
+  const double pl1 = p2fma(2.0, p2fma(-0.0625, f[1], g2), g3);
+  const double pl2 = p2fma(-0.125, f[4], p2fma(2.0, g3, g2));
+  const double u1 = 0.650 * s1;
+  double w0 = 0.075 * s0, w1, w2 = 0.275 * s2;
+  double dn = rcp_normal(w0 + u1 + w2);
+  w0 *= dn;
+  w1 = u1 * dn;
+  w2 = 1.0 - w0 - w1;
+  fl = (+w0 * pl0 + w1 * pl1 + w2 * pl2);
+  const double pr2 = 0.375 * f[4] - 1.25 * f[3] + h2;
+  const double pr1 = p2fma(2.0, p2fma(-0.0625, f[3], g2), g1);
+  const double pr0 = p2fma(-0.125, f[0], p2fma(2.0, g1, g2));
+  w0 = 0.275 * s0;
+  w2 = 0.075 * s2;
+  dn = rcp_normal(w0 + u1 + w2);
+  w0 *= dn;
+  w1 = u1 * dn;
+  w2 = 1.0 - w0 - w1;
+  fr = (+w2 * pr2 + w1 * pr1 + w0 * pr0);
 }
 
 QAS_HD void wcns3_lr(const double f[5], double &fl, double &fr)
@@ -189,6 +287,16 @@ QAS_HD void nl_lr(const double f[5], double &fl, double &fr)
   } else {
     wcns4_lr(f, fl, fr);
   }
+}
+
+// nl_lr in the kernels' form: the 4th order by wcns4_lr_fast (hx: see there)
+template <int ODR>
+QAS_HD void nl_lr_fast(const double f[5], double &fl, double &fr, unsigned &hx)
+{
+  if (ODR == 4)
+    wcns4_lr_fast(f, fl, fr, hx);
+  else
+    nl_lr<ODR>(f, fl, fr);
 }
 
 // ---------------------------------------------------------------------------
@@ -320,118 +428,182 @@ QAS_HD void face_states_prim(const ST &st, double vl[7], double vr[7])
   }
 }
 
+// every value added is zero (either sign), tested by one OR of the bits on the integer pipe
+struct ZeroTest {
+  unsigned long long b = 0;
+  QAS_HD void add(double x)
+  {
+#if defined(__CUDA_ARCH__)
+    b |= (unsigned long long)__double_as_longlong(x);
+#else
+    unsigned long long t;
+    memcpy(&t, &x, 8);
+    b |= t;
+#endif
+  }
+  QAS_HD bool zero() const { return (b << 1) == 0; }
+};
+
 // ---------------------------------------------------------------------------
-// Same reconstruction with the stencil read per characteristic group instead
-// of held in registers: {0,1,2} need ro,vn,bt,bu,pr; {3,4} need vt,bt; {5,6}
-// need vu,bu.  Outputs are accumulated in the reference's term order.
-// `P` is a functor P(v, m) returning primitive v at stencil point m.
+// Same reconstruction in the kernels' form: the stencil is read per characteristic field
+// (`P` is a functor P(v, m) returning primitive v at stencil point m), each component's two
+// states are handed to out(v, left-face-of-the-right-neighbour state, own left-face state)
+// as soon as they are final, and the fields go through one loop body in pairs: {1, 2} (the
+// entropy and the pressure-like row), {3, 4} and {5, 6} (the Alfven rows of either transverse
+// axis); field 0 stands alone.  out.again(P, bn, gam) is called, rarely, where the fast
+// interpolation does not hold, and stores all the states anew by face_states.  Three copies of the interpolation instead of seven keep the
+// code small (the sweeps are held up by instruction fetch) and few values live.
 // ---------------------------------------------------------------------------
-template <int ODR, class Stencil>
-QAS_HD void face_states_grouped(const Stencil &P, double bn, double gam, double vl[7],
-                                                    double vr[7])
+template <int ODR, class Stencil, class Out>
+QAS_HD void face_states_emit(const Stencil &P, double bn, double gam, const Out &out)
 {
-  const double ro = P(0, 2), vn = P(1, 2), vt = P(2, 2), vu = P(3, 2);
-  const double by = P(4, 2), bz = P(5, 2), pr = P(6, 2);
-  const bool fast = (ro * (vn * vn + vt * vt + vu * vu) > gam * pr);
-  double iro = 1.0 / ro;
-  double cs2 = gam * pr * iro;
-  double ca2 = bn * bn * iro;
-  double ct2 = (by * by + bz * bz) * iro;
-  double cb2 = cs2 + ca2 + ct2;
-  double cf2 = 0.5 * (cb2 + sqrt(fabs(cb2 * cb2 - 4.0 * cs2 * ca2)));
-  double sro = sqrt(ro);
-  double isroh = 0.5 / sro;
-  double icf2 = 1.0 / cf2;
-  double byh = 0.5 * by, bzh = 0.5 * bz;
-  double rcf = 0.0, icf2h = 0.0, ircfh = 0.0;
-  if (fast) {
-    double cf = sqrt(cf2);
-    rcf = ro * cf;
-    icf2h = 0.5 * icf2;
-    ircfh = 0.5 / rcf;
+  unsigned hx = 0;
+  double cf2, icf2, sro, isroh, by, bz;
+  bool fast;
+  double l0, r0, l1, r1, l6, r6;  // components 0 (ro), 1 (vn), 6 (pr)
+  {
+    const double ro = P(0, 2), vn = P(1, 2), vt = P(2, 2), vu = P(3, 2), pr = P(6, 2);
+    by = P(4, 2);
+    bz = P(5, 2);
+    fast = (ro * (vn * vn + vt * vt + vu * vu) > gam * pr);
+    const double iro = 1.0 / ro;
+    const double cs2 = gam * pr * iro;
+    const double ca2 = bn * bn * iro;
+    const double ct2 = (by * by + bz * bz) * iro;
+    const double cb2 = cs2 + ca2 + ct2;
+    cf2 = 0.5 * (cb2 + sqrt(fabs(p2fma(-4.0, cs2 * ca2, cb2 * cb2))));
+    sro = sqrt(ro);
+    isroh = 0.5 * (1.0 / sro);
+    icf2 = 1.0 / cf2;
   }
-  const double nrcf = -rcf;
-  bool zvn = true, zvt = true, zvu = true, zbt = true, zbu = true;
-  double wl0, wr0, wl1, wr1, wl2, wr2, wl3, wr3, wl4, wr4, wl5, wr5, wl6, wr6;
-  {  // fast/alfven/entropy group
-    double w0[5], w1[5], w2[5];
+  {  // field 0: vn of the slow eigen-system (mhd_eigen_mi), the backward fast wave of mhd_eigen_ae
+    double w[5];
+    ZeroTest tn;
 #pragma unroll
     for (int m = 0; m < 5; m++) {
-      const double r_ = P(0, m), n_ = P(1, m), b_ = P(4, m), c_ = P(5, m), p_ = P(6, m);
-      zvn = zvn && is_zero(n_);
-      zbt = zbt && is_zero(b_);
-      zbu = zbu && is_zero(c_);
-      w0[m] = fast ? (((nrcf * n_ + by * b_) + bz * c_) + p_) : n_;
-      w1[m] = ((cf2 * r_ - by * b_) - bz * c_) - p_;
-      w2[m] = fast ? (((rcf * n_ + by * b_) + bz * c_) + p_) : ((by * b_ + bz * c_) + p_);
+      w[m] = P(1, m);
+      tn.add(w[m]);
     }
-    nl_lr<ODR>(w0, wl0, wr0);
-    nl_lr<ODR>(w1, wl1, wr1);
-    nl_lr<ODR>(w2, wl2, wr2);
-  }
-  {  // y-Alfven group
-    double w3[5], w4[5];
+    if (fast) {
+      const double rcf = P(0, 2) * sqrt(cf2);
 #pragma unroll
-    for (int m = 0; m < 5; m++) {
-      const double t_ = P(2, m), b_ = P(4, m);
-      zvt = zvt && is_zero(t_);
-      w3[m] = sro * t_ + b_;
-      w4[m] = sro * t_ - b_;
+      for (int m = 0; m < 5; m++) w[m] = (((-rcf) * w[m] + by * P(4, m)) + bz * P(5, m)) + P(6, m);
     }
-    nl_lr<ODR>(w3, wl3, wr3);
-    nl_lr<ODR>(w4, wl4, wr4);
+    nl_lr_fast<ODR>(w, l1, r1, hx);
+    if (!fast && tn.zero()) {
+      l1 = 0.0;
+      r1 = 0.0;
+    }
   }
-  {  // z-Alfven group
-    double w5[5], w6[5];
+#pragma unroll 1
+  for (int g = 0; g < 3; g++) {
+    double wa[5], wb[5], la, ra, lb, rb;
+    ZeroTest tv, tb;
+    if (g == 0) {
 #pragma unroll
-    for (int m = 0; m < 5; m++) {
-      const double u_ = P(3, m), c_ = P(5, m);
-      zvu = zvu && is_zero(u_);
-      w5[m] = sro * u_ + c_;
-      w6[m] = sro * u_ - c_;
+      for (int m = 0; m < 5; m++) {
+        const double p_ = P(6, m), yb = by * P(4, m), zc = bz * P(5, m);
+        wa[m] = ((cf2 * P(0, m) - yb) - zc) - p_;
+        wb[m] = (yb + zc) + p_;
+      }
+      if (fast) {
+        const double rcf = P(0, 2) * sqrt(cf2);
+#pragma unroll
+        for (int m = 0; m < 5; m++) wb[m] = ((rcf * P(1, m) + by * P(4, m)) + bz * P(5, m)) + P(6, m);
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < 5; m++) {
+        const double t_ = P(1 + g, m), b_ = P(3 + g, m);
+        tv.add(t_);
+        tb.add(b_);
+        const double st = sro * t_;
+        wa[m] = st + b_;
+        wb[m] = st - b_;
+      }
     }
-    nl_lr<ODR>(w5, wl5, wr5);
-    nl_lr<ODR>(w6, wl6, wr6);
+    nl_lr_fast<ODR>(wa, la, ra, hx);
+    nl_lr_fast<ODR>(wb, lb, rb, hx);
+    if (g == 0) {
+      if (fast) {
+        const double icf2h = 0.5 * icf2, ircfh = 0.5 / (P(0, 2) * sqrt(cf2));
+        l0 = icf2h * l1 + icf2 * la + icf2h * lb;
+        r0 = icf2h * r1 + icf2 * ra + icf2h * rb;
+        l6 = 0.5 * (l1 + lb);
+        r6 = 0.5 * (r1 + rb);
+        l1 = (-ircfh) * l1 + ircfh * lb;
+        r1 = (-ircfh) * r1 + ircfh * rb;
+        ZeroTest tn;
+#pragma unroll
+        for (int m = 0; m < 5; m++) tn.add(P(1, m));
+        if (tn.zero()) {
+          l1 = 0.0;
+          r1 = 0.0;
+        }
+      } else {
+        l0 = icf2 * la + icf2 * lb;
+        r0 = icf2 * ra + icf2 * rb;
+        l6 = lb;
+        r6 = rb;
+      }
+    } else {
+      const double bh = 0.5 * (g == 1 ? by : bz);
+      l6 = (l6 - bh * la) + bh * lb;
+      r6 = (r6 - bh * ra) + bh * rb;
+      const bool zv = tv.zero(), zb = tb.zero();  // exactly-zero fields stay exactly zero
+      out(1 + g, zv ? 0.0 : isroh * la + isroh * lb, zv ? 0.0 : isroh * ra + isroh * rb);
+      out(3 + g, zb ? 0.0 : 0.5 * (la - lb), zb ? 0.0 : 0.5 * (ra - rb));
+    }
   }
-  if (fast) {
-    vl[0] = icf2h * wl0 + icf2 * wl1 + icf2h * wl2;
-    vr[0] = icf2h * wr0 + icf2 * wr1 + icf2h * wr2;
-    vl[1] = (-ircfh) * wl0 + ircfh * wl2;
-    vr[1] = (-ircfh) * wr0 + ircfh * wr2;
-    vl[6] = ((((0.5 * wl0 + 0.5 * wl2) - byh * wl3) + byh * wl4) - bzh * wl5) + bzh * wl6;
-    vr[6] = ((((0.5 * wr0 + 0.5 * wr2) - byh * wr3) + byh * wr4) - bzh * wr5) + bzh * wr6;
-  } else {
-    vl[0] = icf2 * wl1 + icf2 * wl2;
-    vr[0] = icf2 * wr1 + icf2 * wr2;
-    vl[1] = wl0;
-    vr[1] = wr0;
-    vl[6] = (((wl2 - byh * wl3) + byh * wl4) - bzh * wl5) + bzh * wl6;
-    vr[6] = (((wr2 - byh * wr3) + byh * wr4) - bzh * wr5) + bzh * wr6;
+  const double eps = 1e-12;  // positivity fallback to first order (mhd_func.c:150-160)
+  if (l0 <= eps || l6 <= eps) {
+    l0 = P(0, 2);
+    l1 = P(1, 2);
+    l6 = P(6, 2);
   }
-  vl[2] = isroh * wl3 + isroh * wl4;
-  vr[2] = isroh * wr3 + isroh * wr4;
-  vl[3] = isroh * wl5 + isroh * wl6;
-  vr[3] = isroh * wr5 + isroh * wr6;
-  vl[4] = 0.5 * wl3 - 0.5 * wl4;
-  vr[4] = 0.5 * wr3 - 0.5 * wr4;
-  vl[5] = 0.5 * wl5 - 0.5 * wl6;
-  vr[5] = 0.5 * wr5 - 0.5 * wr6;
-  if (zvn) { vl[1] = 0.0; vr[1] = 0.0; }
-  if (zvt) { vl[2] = 0.0; vr[2] = 0.0; }
-  if (zvu) { vl[3] = 0.0; vr[3] = 0.0; }
-  if (zbt) { vl[4] = 0.0; vr[4] = 0.0; }
-  if (zbu) { vl[5] = 0.0; vr[5] = 0.0; }
-  const double eps = 1e-12;
-  if (vl[0] <= eps || vl[6] <= eps) {
-    vl[0] = ro;
-    vl[1] = vn;
-    vl[6] = pr;
+  if (r0 <= eps || r6 <= eps) {
+    r0 = P(0, 2);
+    r1 = P(1, 2);
+    r6 = P(6, 2);
   }
-  if (vr[0] <= eps || vr[6] <= eps) {
-    vr[0] = ro;
-    vr[1] = vn;
-    vr[6] = pr;
+  out(0, l0, r0);
+  out(1, l1, r1);
+  out(6, l6, r6);
+  // a smoothness denominator beyond 2^900 or a NaN: all over again with the reference's divisions
+  if (ODR == 4 && hx >= WCNS_HX) out.again(P, bn, gam);
+}
+
+// face_states from a stencil functor
+template <int ODR, class Stencil>
+QAS_HD void face_states_of(const Stencil &P, double bn, double gam, double vl[7], double vr[7])
+{
+  double q[7][5];
+#pragma unroll
+  for (int f = 0; f < 7; f++)
+#pragma unroll
+    for (int m = 0; m < 5; m++) q[f][m] = P(f, m);
+  face_states<ODR>(q, bn, gam, vl, vr);
+}
+
+// the same into arrays
+template <int ODR>
+struct StatesInto {
+  double *vl, *vr;
+  QAS_HD void operator()(int m, double l, double r) const
+  {
+    vl[m] = l;
+    vr[m] = r;
   }
+  template <class Stencil>
+  QAS_HD void again(const Stencil &P, double bn, double gam) const
+  {
+    face_states_of<ODR>(P, bn, gam, vl, vr);
+  }
+};
+template <int ODR, class Stencil>
+QAS_HD void face_states_grouped(const Stencil &P, double bn, double gam, double vl[7], double vr[7])
+{
+  face_states_emit<ODR>(P, bn, gam, StatesInto<ODR>{vl, vr});
 }
 
 // ---------------------------------------------------------------------------
@@ -569,46 +741,49 @@ QAS_HD void face_states_athena(const Stencil &P, double bx, double gamma, double
 // ---------------------------------------------------------------------------
 #define QAS_FL_EPS (1e-8)
 
-// HLLD (LOW=false, mhd_flux.c:435-561) and low-dissipation LHLLD (LOW=true, :563-698)
+// cb + sqrt(|cb^2 - 4 x ca|), the larger of the two sides (twice the squared speed of the faster
+// side): the sum and the root are monotonic also after rounding, so where one side has both the
+// larger cb and the larger discriminant its root alone is taken; the second root only where the
+// two disagree
+QAS_HD double larger_speed2(double cbl, double xl, double cal, double cbr, double xr, double car)
+{
+  const double dl = fabs(p2fma(-4.0, xl * cal, cbl * cbl)), dr = fabs(p2fma(-4.0, xr * car, cbr * cbr));
+  const bool left = cbl >= cbr;
+  const double cb = left ? cbl : cbr, d = left ? dl : dr, co = left ? cbr : cbl, o = left ? dr : dl;
+  const double f = cb + sqrt(d);
+  if (d >= o) return f;
+  return qmax(f, co + sqrt(o));  // a NaN on either side comes here too
+}
+
+// HLLD (LOW=false, mhd_flux.c:435-561) and low-dissipation LHLLD (LOW=true, :563-698).
+// The reference forms all four star states of both sides and adds them with weights of exactly 0
+// or 1; here the side of the contact (vnc > 0) and the outer / inner state are chosen first and
+// only that side's energy, Alfven-wave speed and products are formed (each by the reference's
+// expression): two IEEE divisions and about a third of the FP64 work less.  A weighted sum and
+// the choice differ only where an unused state is not finite, which needs a face state with
+// ro <= 0 or pr <= 0 (sl < vnc < sr otherwise).
 template <bool LOW>
-QAS_HD void flux_hlld(const double L[7], const double R[7], double bnc, double gamma,
+QAS_HD void flux_hlld(const double L[7], const double R[7], double bnc, double gamma, double gammam1i,
                                           double dv0, double dv1, double F[7])
 {
   const double rol = L[0], vnl = L[1], vtl = L[2], vul = L[3], btl = L[4], bul = L[5], prl = L[6];
   const double ror = R[0], vnr = R[1], vtr = R[2], vur = R[3], btr = R[4], bur = R[5], prr = R[6];
-  double gammam1i = 1.0 / (gamma - 1.0);
-  double bnc2 = bnc * bnc;
-  double sgn = (bnc > 0) ? (1.0) : (-1.0);
-  double roli = 1.0 / rol;
-  double vl2 = vnl * vnl + vtl * vtl + vul * vul;
-  double pml = 0.5 * (btl * btl + bul * bul);
-  double ptl = prl + pml;
-  double enl = gammam1i * prl + pml + 0.5 * rol * vl2;
-  double vbl = vtl * btl + vul * bul;
-  double rori = 1.0 / ror;
-  double vr2 = vnr * vnr + vtr * vtr + vur * vur;
-  double pmr = 0.5 * (btr * btr + bur * bur);
-  double ptr = prr + pmr;
-  double enr = gammam1i * prr + pmr + 0.5 * ror * vr2;
-  double vbr = vtr * btr + vur * bur;
-  double cl2 = gamma * prl * roli;
-  double cr2 = gamma * prr * rori;
-  double cal2 = bnc2 * roli;
-  double car2 = bnc2 * rori;
-  double cbl2 = cl2 + cal2 + 2.0 * pml * roli;
-  double cbr2 = cr2 + car2 + 2.0 * pmr * rori;
-  double cfl2 = 0.5 * (cbl2 + sqrt(fabs(cbl2 * cbl2 - 4.0 * cl2 * cal2)));
-  double cfr2 = 0.5 * (cbr2 + sqrt(fabs(cbr2 * cbr2 - 4.0 * cr2 * car2)));
-  double cmax, ccl2 = 0.0, ccr2 = 0.0;
-  if (LOW) {
-    cbl2 = vl2 + cal2 + 2.0 * pml * roli;
-    cbr2 = vr2 + car2 + 2.0 * pmr * rori;
-    ccl2 = 0.5 * (cbl2 + sqrt(fabs(cbl2 * cbl2 - 4.0 * vl2 * cal2)));
-    ccr2 = 0.5 * (cbr2 + sqrt(fabs(cbr2 * cbr2 - 4.0 * vr2 * car2)));
-    cmax = sqrt(qmax(cfl2, cfr2));
-  } else {
-    cmax = qmax(sqrt(cfl2), sqrt(cfr2));
-  }
+  const double bnc2 = bnc * bnc;
+  const bool neg = !(bnc > 0);  // sgn = -1
+  const double roli = 1.0 / rol;
+  const double bl2 = btl * btl + bul * bul;  // 2 pml
+  const double ptl = p2fma(0.5, bl2, prl);
+  const double rori = 1.0 / ror;
+  const double br2 = btr * btr + bur * bur;
+  const double ptr = p2fma(0.5, br2, prr);
+  const double vl2 = vnl * vnl + vtl * vtl + vul * vul;
+  const double vr2 = vnr * vnr + vtr * vtr + vur * vur;
+  const double cl2 = gamma * prl * roli;
+  const double cr2 = gamma * prr * rori;
+  const double cal2 = bnc2 * roli;
+  const double car2 = bnc2 * rori;
+  const double tl = bl2 * roli, tr = br2 * rori;
+  const double cmax = sqrt(0.5 * larger_speed2(cl2 + cal2 + tl, cl2, cal2, cr2 + car2 + tr, cr2, car2));
   double sl = qmin(0.0, qmin(vnl, vnr) - cmax);
   double sr = qmax(0.0, qmax(vnl, vnr) + cmax);
   double slvl = sl - vnl;
@@ -622,7 +797,8 @@ QAS_HD void flux_hlld(const double L[7], const double R[7], double bnc, double g
     theta *= theta;
     theta *= theta;
     vnc = (rsrvr * vnr - rslvl * vnl - theta * (ptr - ptl)) * drsvi;
-    double mcc = qmin(1.0, sqrt(qmax(ccl2, ccr2)) / cmax);
+    const double cc = larger_speed2(vl2 + cal2 + tl, vl2, cal2, vr2 + car2 + tr, vr2, car2);
+    double mcc = qmin(1.0, sqrt(0.5 * cc) / cmax);
     ptc = (rsrvr * ptl - rslvl * ptr + (mcc * (2.0 - mcc)) * rsrvr * rslvl * (vnr - vnl)) * drsvi;
   } else {
     vnc = (rsrvr * vnr - rslvl * vnl - ptr + ptl) * drsvi;
@@ -639,10 +815,11 @@ QAS_HD void flux_hlld(const double L[7], const double R[7], double bnc, double g
     double rhdli = 1.0 / rhdl;
     double rhnvl = (vnl - vnc) * bnc;
     double rhnbl = rslvl * slvl - bnc2;
-    vt2l = vtl + rhnvl * rhdli * btl;
-    vu2l = vul + rhnvl * rhdli * bul;
-    bt2l = rhnbl * rhdli * btl;
-    bu2l = rhnbl * rhdli * bul;
+    const double av = rhnvl * rhdli, ab = rhnbl * rhdli;
+    vt2l = vtl + av * btl;
+    vu2l = vul + av * bul;
+    bt2l = ab * btl;
+    bu2l = ab * bul;
   } else {
     vt2l = vtl; vu2l = vul; bt2l = btl; bu2l = bul;
   }
@@ -650,41 +827,48 @@ QAS_HD void flux_hlld(const double L[7], const double R[7], double bnc, double g
     double rhdri = 1.0 / rhdr;
     double rhnvr = (vnr - vnc) * bnc;
     double rhnbr = rsrvr * srvr - bnc2;
-    vt2r = vtr + rhnvr * rhdri * btr;
-    vu2r = vur + rhnvr * rhdri * bur;
-    bt2r = rhnbr * rhdri * btr;
-    bu2r = rhnbr * rhdri * bur;
+    const double av = rhnvr * rhdri, ab = rhnbr * rhdri;
+    vt2r = vtr + av * btr;
+    vu2r = vur + av * bur;
+    bt2r = ab * btr;
+    bu2r = ab * bur;
   } else {
     vt2r = vtr; vu2r = vur; bt2r = btr; bu2r = bur;
   }
-  double vb2l = vt2l * bt2l + vu2l * bu2l;
-  double vb2r = vt2r * bt2r + vu2r * bu2r;
-  double en2l = (slvl * enl - ptl * vnl + ptc * vnc + bnc * (vbl - vb2l)) / slvc;
-  double en2r = (srvr * enr - ptr * vnr + ptc * vnc + bnc * (vbr - vb2r)) / srvc;
-  double rro2l = sqrt(ro2l);
-  double rro2r = sqrt(ro2r);
-  double rro2i = 1.0 / (rro2r + rro2l);
-  double vt3m = (rro2r * vt2r + rro2l * vt2l + (bt2r - bt2l) * sgn) * rro2i;
-  double vu3m = (rro2r * vu2r + rro2l * vu2l + (bu2r - bu2l) * sgn) * rro2i;
-  double bt3m = (rro2l * bt2r + rro2r * bt2l + rro2r * rro2l * (vt2r - vt2l) * sgn) * rro2i;
-  double bu3m = (rro2l * bu2r + rro2r * bu2l + rro2r * rro2l * (vu2r - vu2l) * sgn) * rro2i;
-  double vb3m = vt3m * bt3m + vu3m * bu3m;
-  double en3l = en2l - rro2l * (vb2l - vb3m) * sgn;
-  double en3r = en2r + rro2r * (vb2r - vb3m) * sgn;
-  double hl = (vnc > 0) ? (1.0) : (0.0);
-  double hr = 1.0 - hl;
-  double h2l = (vnc - fabs(bnc) / rro2l > 0) ? (1.0) : (0.0);
-  double h3l = (1.0 - h2l) * hl;
-  double h2r = (vnc + fabs(bnc) / rro2r > 0) ? (0.0) : (1.0);
-  double h3r = (1.0 - h2r) * hr;
-  double rou = ro2l * hl + ro2r * hr;
-  double vtu = vt2l * h2l + vt3m * (h3l + h3r) + vt2r * h2r;
-  double vuu = vu2l * h2l + vu3m * (h3l + h3r) + vu2r * h2r;
-  double btu = bt2l * h2l + bt3m * (h3l + h3r) + bt2r * h2r;
-  double buu = bu2l * h2l + bu3m * (h3l + h3r) + bu2r * h2r;
-  double enu = en2l * h2l + en3l * h3l + en3r * h3r + en2r * h2r;
-  F[0] = rou * vnc;
-  F[1] = rou * vnc * vnc + ptc - bnc2 * 0.5;
+  const double rro2l = sqrt(ro2l);
+  const double rro2r = sqrt(ro2r);
+  const double rro2i = 1.0 / (rro2r + rro2l);
+  const bool left = vnc > 0;
+  // the upwind side
+  const double ro_ = left ? rol : ror, vn_ = left ? vnl : vnr, vt_ = left ? vtl : vtr, vu_ = left ? vul : vur;
+  const double bt_ = left ? btl : btr, bu_ = left ? bul : bur, pr_ = left ? prl : prr, pt_ = left ? ptl : ptr;
+  const double b2_ = left ? bl2 : br2, v2_ = left ? vl2 : vr2, sv_ = left ? slvl : srvr, sc_ = left ? slvc : srvc;
+  const double vt2 = left ? vt2l : vt2r, vu2 = left ? vu2l : vu2r;
+  const double bt2 = left ? bt2l : bt2r, bu2 = left ? bu2l : bu2r;
+  const double rro2 = left ? rro2l : rro2r;
+  const double en = p2fma(0.5, ro_ * v2_, p2fma(0.5, b2_, gammam1i * pr_));
+  const double vb = vt_ * bt_ + vu_ * bu_;
+  const double vb2 = vt2 * bt2 + vu2 * bu2;
+  const double en2 = (sv_ * en - pt_ * vn_ + ptc * vnc + bnc * (vb - vb2)) / sc_;
+  const double ca = fabs(bnc) / rro2;
+  const bool outer = left ? (vnc - ca > 0) : !(vnc + ca > 0);
+  const double vt3m = (rro2r * vt2r + rro2l * vt2l + flip(bt2r - bt2l, neg)) * rro2i;
+  const double vu3m = (rro2r * vu2r + rro2l * vu2l + flip(bu2r - bu2l, neg)) * rro2i;
+  const double rr = rro2r * rro2l;
+  const double bt3m = (rro2l * bt2r + rro2r * bt2l + flip(rr * (vt2r - vt2l), neg)) * rro2i;
+  const double bu3m = (rro2l * bu2r + rro2r * bu2l + flip(rr * (vu2r - vu2l), neg)) * rro2i;
+  const double vb3m = vt3m * bt3m + vu3m * bu3m;
+  // en2 - rro2*(vb2 - vb3)*sgn on the left, + on the right
+  const double en3 = en2 + flip(rro2 * (vb2 - vb3m), neg != left);
+  const double rou = left ? ro2l : ro2r;
+  const double vtu = outer ? vt2 : vt3m;
+  const double vuu = outer ? vu2 : vu3m;
+  const double btu = outer ? bt2 : bt3m;
+  const double buu = outer ? bu2 : bu3m;
+  const double enu = outer ? en2 : en3;
+  const double mf = rou * vnc;
+  F[0] = mf;
+  F[1] = p2fma(-0.5, bnc2, mf * vnc + ptc);
   F[2] = rou * vtu * vnc - bnc * btu;
   F[3] = rou * vuu * vnc - bnc * buu;
   F[4] = btu * vnc - bnc * vtu;
@@ -693,128 +877,116 @@ QAS_HD void flux_hlld(const double L[7], const double R[7], double bnc, double g
 }
 
 // MLAU all-speed flux, common/mhd_flux.c:7-192.  Every value keeps the reference's expression
-// and operation order; only the order of independent statements differs, so that few values are
-// live at once (the kernels run this solver at 80 registers): the first two energy-flux terms are
-// summed as soon as their factors exist, the two transverse components are finished one after
-// the other, and each flux goes to out(m, value) as soon as it is final (the kernels store it at
-// once).  out receives F = (fro, fmn, fmt, fmu, fbt, fbu, fen) in the order 0, 1, 2, 4, 3, 5, 6.
+// and rounding; what differs is which values are formed.  The reference weighs the two sides with
+// dirl, dirr = (1, 0) or (0, 1); here the upwind side's operands are chosen and only its energy,
+// products and sums are formed, products by +-1 are sign flips, and the larger of two speeds takes
+// one square root where it can (larger_speed2).  Few values are live at once (the kernels run this
+// solver at 80 registers): the two transverse components are finished one after the other, and
+// each flux goes to out(m, value) as soon as it is final (the kernels store it at once).  out
+// receives F = (fro, fmn, fmt, fmu, fbt, fbu, fen) in the order 0, 1, 2, 4, 3, 5, 6.
 template <class Out>
-QAS_HD void flux_mlau_out(const double L[7], const double R[7], double bnc, double gamma, double dv0, double dv1,
-                          Out &&out)
+QAS_HD void flux_mlau_out(const double L[7], const double R[7], double bnc, double gamma, double gammam1i, double dv0,
+                          double dv1, Out &&out)
 {
   const double rol = L[0], vnl = L[1], vtl = L[2], vul = L[3], btl = L[4], bul = L[5], prl = L[6];
   const double ror = R[0], vnr = R[1], vtr = R[2], vur = R[3], btr = R[4], bur = R[5], prr = R[6];
-  double gammam1i = 1.0 / (gamma - 1.0);
-  double bnc2 = bnc * bnc;
-  double sgn = (bnc > 0) ? (1.0) : (-1.0);
-  double bnca = sgn * bnc;
-  double roli = 1.0 / rol;
-  double vl2 = vnl * vnl + vtl * vtl + vul * vul;
-  double pml = 0.5 * (btl * btl + bul * bul);
-  double ptl = prl + pml;
-  double enl = gammam1i * prl + pml + 0.5 * rol * vl2;
-  double hnl = (enl + ptl) * roli;
-  double rori = 1.0 / ror;
-  double vr2 = vnr * vnr + vtr * vtr + vur * vur;
-  double pmr = 0.5 * (btr * btr + bur * bur);
-  double ptr = prr + pmr;
-  double enr = gammam1i * prr + pmr + 0.5 * ror * vr2;
-  double hnr = (enr + ptr) * rori;
-  double cl2 = gamma * prl * roli;
-  double cr2 = gamma * prr * rori;
-  double cal2 = bnc2 * roli;
-  double car2 = bnc2 * rori;
-  double cbl2 = cl2 + cal2 + 2.0 * pml * roli;
-  double cbr2 = cr2 + car2 + 2.0 * pmr * rori;
-  double cfl2 = 0.5 * (cbl2 + sqrt(fabs(cbl2 * cbl2 - 4.0 * cl2 * cal2)));
-  double cfr2 = 0.5 * (cbr2 + sqrt(fabs(cbr2 * cbr2 - 4.0 * cr2 * car2)));
-  cbl2 = vl2 + cal2 + 2.0 * pml * roli;
-  cbr2 = vr2 + car2 + 2.0 * pmr * rori;
-  double ccl2 = 0.5 * (cbl2 + sqrt(fabs(cbl2 * cbl2 - 4.0 * vl2 * cal2)));
-  double ccr2 = 0.5 * (cbr2 + sqrt(fabs(cbr2 * cbr2 - 4.0 * vr2 * car2)));
-  double cmax = sqrt(qmax(cfl2, cfr2));
-  double cfmod = sqrt(qmax(ccl2, ccr2));
-  double cfn = cmax;
-  double cfni = 1.0 / cfn;
-  double sl = qmin(0.0, qmin(vnl, vnr) - cmax);
-  double sr = qmax(0.0, qmax(vnl, vnr) + cmax);
-  double mal = vnl * cfni;
-  double mar = vnr * cfni;
-  double snl = (mal > 0) ? 1.0 : (-1.0);
-  double snr = (mar > 0) ? 1.0 : (-1.0);
+  const double bnc2 = bnc * bnc;
+  const bool neg = !(bnc > 0);  // sgn = -1
+  const double bnca = flip(bnc, neg);
+  const double roli = 1.0 / rol;
+  const double vl2 = vnl * vnl + vtl * vtl + vul * vul;
+  const double bl2 = btl * btl + bul * bul;  // 2 pml
+  const double ptl = p2fma(0.5, bl2, prl);
+  const double rori = 1.0 / ror;
+  const double vr2 = vnr * vnr + vtr * vtr + vur * vur;
+  const double br2 = btr * btr + bur * bur;
+  const double ptr = p2fma(0.5, br2, prr);
+  double cfn, cfmod;
+  {
+    const double cl2 = gamma * prl * roli, cr2 = gamma * prr * rori;
+    const double cal2 = bnc2 * roli, car2 = bnc2 * rori;
+    const double tl = bl2 * roli, tr = br2 * rori;
+    cfn = sqrt(0.5 * larger_speed2(cl2 + cal2 + tl, cl2, cal2, cr2 + car2 + tr, cr2, car2));
+    cfmod = sqrt(0.5 * larger_speed2(vl2 + cal2 + tl, vl2, cal2, vr2 + car2 + tr, vr2, car2));
+  }
+  const double cfni = 1.0 / cfn;
+  const double sl = qmin(0.0, qmin(vnl, vnr) - cfn);
+  const double sr = qmax(0.0, qmax(vnl, vnr) + cfn);
+  const double mal = vnl * cfni;
+  const double mar = vnr * cfni;
   double theta = qmin(1.0, (cfn - qmin(dv0, 0.0)) / (cfn - qmin(dv1, 0.0)));
   theta *= theta;
   theta *= theta;
-  const double alpha = 0.1875, beta = 0.125;
-  double malp1 = mal + 1.0;
-  double marm1 = mar - 1.0;
-  double mal2m1 = mal * mal - 1.0;
-  double mar2m1 = mar * mar - 1.0;
+  const double alpha = 0.1875;
   double bfl, ffl, bfr, ffr;
-  if (snl * mal > 1.0) {
-    bfl = 0.5 * (1.0 + snl);
+  if (fabs(mal) > 1.0) {
+    bfl = mal > 0 ? 1.0 : 0.0;
     ffl = bfl * mal;
   } else {
-    bfl = +0.25 * malp1 * malp1 * (2.0 - mal) + alpha * mal * mal2m1 * mal2m1;
-    ffl = +0.25 * malp1 * malp1 + beta * mal2m1 * mal2m1;
+    const double p1 = mal + 1.0, m1 = mal * mal - 1.0, pp = p1 * p1, mm = m1 * m1;
+    bfl = p2fma(0.25, pp * (2.0 - mal), alpha * mal * m1 * m1);
+    ffl = p2fma(0.25, pp, 0.125 * mm);
   }
-  if (snr * mar > 1.0) {
-    bfr = 0.5 * (1.0 - snr);
+  if (fabs(mar) > 1.0) {
+    bfr = mar > 0 ? 0.0 : 1.0;
     ffr = bfr * mar;
   } else {
-    bfr = +0.25 * marm1 * marm1 * (2.0 + mar) - alpha * mar * mar2m1 * mar2m1;
-    ffr = -0.25 * marm1 * marm1 - beta * mar2m1 * mar2m1;
+    const double p1 = mar - 1.0, m1 = mar * mar - 1.0, pp = p1 * p1, mm = m1 * m1;
+    bfr = p2fma(0.25, pp * (2.0 + mar), -(alpha * mar * m1 * m1));
+    ffr = p2fma(-0.25, pp, -(0.125 * mm));
   }
-  double mnc = ffl + ffr;
+  const double mnc = ffl + ffr;
   double mflux = mnc * cfn;
   mflux -= qmax(1.0 - fabs(mnc), 0.0) * theta * cfni * (ptr - ptl) / (rol + ror);
-  double dir = (mflux > 0) ? 1.0 : (-1.0);
-  double dirl = 0.5 * (1.0 + dir);
-  double dirr = 1.0 - dirl;
-  mflux *= (dirl * rol + dirr * ror);
+  const bool up = mflux > 0;  // the left side is upwind: dirl = 1, dirr = 0
+  mflux *= up ? rol : ror;
   out(0, mflux);
-  double mfl = mflux * dirl;
-  double mfr = mflux - mfl;
-  double ptot = bfl * ptl + bfr * ptr;
-  ptot -= 0.25 * bfl * bfr * (rol + ror) * cfmod * (vnr - vnl);
-  ptot -= 0.5 * (1.0 - cfmod * cfni) * (bfl + bfr - 1.0) * (ptl + ptr);
-  out(1, mfl * vnl + mfr * vnr + ptot - 0.5 * bnc2);
-  const double e6 = mfl * hnl + mfr * hnr;  // fen = e6 - bnvb
-  double slvl = sl - vnl;
-  double srvr = sr - vnr;
-  double snc = dirl * sl + dirr * sr;
-  double vndnm = mflux + dirl * rol * slvl + dirr * ror * srvr;
-  double vnc = ((fabs(vndnm) > QAS_FL_EPS) && (snc != 0)) ? (mflux * snc / vndnm) : (dirl * vnl + dirr * vnr);
-  double slvc = sl - vnc;
-  double srvc = sr - vnc;
-  double slvci = 1.0 / slvc;
-  double srvci = 1.0 / srvc;
-  double rhdl = rol * slvl * slvc - bnc2;
-  double rhdr = ror * srvr * srvc - bnc2;
+  {
+    double ptot = bfl * ptl + bfr * ptr;
+    ptot = p2fma(-0.25, bfl * bfr * (rol + ror) * cfmod * (vnr - vnl), ptot);
+    ptot = p2fma(-0.5, (1.0 - cfmod * cfni) * (bfl + bfr - 1.0) * (ptl + ptr), ptot);
+    out(1, p2fma(-0.5, bnc2, mflux * (up ? vnl : vnr) + ptot));
+  }
+  const double roui = up ? roli : rori;
+  double e6;  // fen = e6 - bnvb
+  {
+    const double en = p2fma(0.5, (up ? rol : ror) * (up ? vl2 : vr2),
+                            p2fma(0.5, up ? bl2 : br2, gammam1i * (up ? prl : prr)));
+    e6 = mflux * ((en + (up ? ptl : ptr)) * roui);
+  }
+  const double slvl = sl - vnl;
+  const double srvr = sr - vnr;
+  const double snc = up ? sl : sr;
+  const double rsl = rol * slvl, rsr = ror * srvr;
+  const double vndnm = mflux + (up ? rsl : rsr);
+  const double vnc = ((fabs(vndnm) > QAS_FL_EPS) && (snc != 0)) ? (mflux * snc / vndnm) : (up ? vnl : vnr);
+  const double slvc = sl - vnc;
+  const double srvc = sr - vnc;
+  const double slvci = 1.0 / slvc;
+  const double srvci = 1.0 / srvc;
+  const double rhdl = rsl * slvc - bnc2;
+  const double rhdr = rsr * srvc - bnc2;
   // the reference's q of each side, used only where |rhd| > FL_EPS (else the corrections are 0.0)
   const bool hl = fabs(rhdl) > QAS_FL_EPS, hr = fabs(rhdr) > QAS_FL_EPS;
   const double ql = hl ? (vnc - vnl) / rhdl : 0.0;
   const double qr = hr ? (vnc - vnr) / rhdr : 0.0;
-  double cmpl = slvl * slvci;
-  double cmpr = srvr * srvci;
-  double ro2l = rol * cmpl;
-  double srol = sqrt(ro2l);
-  double ro2r = ror * cmpr;
-  double sror = sqrt(ro2r);
-  double sroi = 1.0 / (srol + sror);
-  double srollri = srol * sroi;
-  double srorlri = sror * sroi;
-  double bnflb = sgn * qmin(qmax(0.0, srollri * (bnca + sror * vnc)), bnca);
-  double bnfrb = sgn * qmin(qmax(0.0, srorlri * (bnca - srol * vnc)), bnca);
-  double bnflv = sgn * qmin(qmax(0.0, srorlri * (bnca + mflux / sror)), bnca);
-  double bnfrv = sgn * qmin(qmax(0.0, srollri * (bnca - mflux / srol)), bnca);
-  double bnsrv = qmax(bnca - dir * vnc * (dirl * srol + dirr * sror), 0.0);
-  double ccb = sroi * bnsrv;
-  double ccv = srol * sror * ccb;
-  double vb1 = dirl * (vtl * btl + vul * bul) + dirr * (vtr * btr + vur * bur);
+  const double cmpl = slvl * slvci;
+  const double cmpr = srvr * srvci;
+  const double srol = sqrt(rol * cmpl);
+  const double sror = sqrt(ror * cmpr);
+  const double sroi = 1.0 / (srol + sror);
+  const double srollri = srol * sroi;
+  const double srorlri = sror * sroi;
+  const double bnflb = flip(qmin(qmax(0.0, srollri * (bnca + sror * vnc)), bnca), neg);
+  const double bnfrb = flip(qmin(qmax(0.0, srorlri * (bnca - srol * vnc)), bnca), neg);
+  const double bnflv = flip(qmin(qmax(0.0, srorlri * (bnca + mflux / sror)), bnca), neg);
+  const double bnfrv = flip(qmin(qmax(0.0, srollri * (bnca - mflux / srol)), bnca), neg);
+  const double bnsrv = qmax(bnca - flip(vnc * (up ? srol : sror), !up), 0.0);
+  const double ccb = sroi * bnsrv;
+  const double ccv = srol * sror * ccb;
   // one transverse component (t: vt, bt; u: vu, bu): its momentum and induction fluxes, its
-  // terms of vb2 (v2*b2 of each side) and its term of vb3's numerator
-  auto comp = [&](double vl_, double bl_, double vr_, double br_, int mf, int mb, double &pl, double &pr,
+  // terms of vb1 and vb2 (v*b of the upwind side) and of vb3's numerator
+  auto comp = [&](double vl_, double bl_, double vr_, double br_, int mf, int mb, double &p1, double &p2,
                   double &q3) {
     const double dvl = hl ? -bnc * bl_ * ql : 0.0;
     const double dbl = hl ? bnc2 * bl_ * ql * slvci : 0.0;
@@ -824,44 +996,49 @@ QAS_HD void flux_mlau_out(const double L[7], const double R[7], double bnc, doub
     const double b2l = dbl + bl_ * cmpl;
     const double v2r = dvr + vr_;
     const double b2r = dbr + br_ * cmpr;
+    const double vu_ = up ? vl_ : vr_, bu_ = up ? bl_ : br_;
     double bnv = bnflb * v2l + bnfrb * v2r + ccb * (b2r - b2l);
     double bnb = bnflv * b2l + bnfrv * b2r + ccv * (v2r - v2l);
-    bnv -= vnc * (dirl * dbl + dirr * dbr);
-    bnb -= mflux * (dirl * dvl + dirr * dvr);
-    const double fm = mfl * vl_ + mfr * vr_ - bnb;
-    const double fb = mfl * bl_ * roli + mfr * br_ * rori - bnv;
+    bnv -= vnc * (up ? dbl : dbr);
+    bnb -= mflux * (up ? dvl : dvr);
+    const double fm = mflux * vu_ - bnb;
+    const double fb = mflux * bu_ * roui - bnv;
     out(mf, fm);
     out(mb, fb);
-    pl = v2l * b2l;
-    pr = v2r * b2r;
+    p1 = vu_ * bu_;
+    p2 = (up ? v2l : v2r) * (up ? b2l : b2r);
     q3 = (fm * vnc + fb * bnc) * (fm * bnc + fb * mflux);
   };
-  double plt, prt, q3t, plu, pru, q3u;
-  comp(vtl, btl, vtr, btr, 2, 4, plt, prt, q3t);
-  comp(vul, bul, vur, bur, 3, 5, plu, pru, q3u);
-  double vb2 = dirl * (plt + plu) + dirr * (prt + pru);
+  double vb1 = 0.0, vb2 = 0.0, q3 = 0.0;
+#pragma unroll
+  for (int t = 0; t < 2; t++) {
+    double p1, p2, q;
+    comp(t == 0 ? vtl : vul, t == 0 ? btl : bul, t == 0 ? vtr : vur, t == 0 ? btr : bur, 2 + t, 4 + t, p1, p2, q);
+    vb1 = t == 0 ? p1 : vb1 + p1;
+    vb2 = t == 0 ? p2 : vb2 + p2;
+    q3 = t == 0 ? q : q3 + q;
+  }
   double rv2b2 = (mflux * vnc - bnc2);
   rv2b2 *= rv2b2;
   double vb3 = 0.0;
-  if (rv2b2 > QAS_FL_EPS * QAS_FL_EPS) vb3 = (q3t + q3u) / rv2b2;
-  double bnvb = sgn * (bnca * (snc * vb2 - vnc * vb1) * (dirl * slvci + dirr * srvci) + bnsrv * (vb3 - vb2));
+  if (rv2b2 > QAS_FL_EPS * QAS_FL_EPS) vb3 = q3 / rv2b2;
+  const double bnvb = flip(bnca * (snc * vb2 - vnc * vb1) * (up ? slvci : srvci) + bnsrv * (vb3 - vb2), neg);
   out(6, e6 - bnvb);
 }
 
-QAS_HD void flux_mlau(const double L[7], const double R[7], double bnc, double gamma, double dv0, double dv1,
-                      double F[7])
+QAS_HD void flux_mlau(const double L[7], const double R[7], double bnc, double gamma, double gammam1i, double dv0,
+                      double dv1, double F[7])
 {
-  flux_mlau_out(L, R, bnc, gamma, dv0, dv1, [&](int m, double x) { F[m] = x; });
+  flux_mlau_out(L, R, bnc, gamma, gammam1i, dv0, dv1, [&](int m, double x) { F[m] = x; });
 }
 
 // Roe flux, common/mhd_flux.c:194-433
-QAS_HD void flux_roe(const double L[7], const double R[7], double bnc, double gamma, double F[7])
+QAS_HD void flux_roe(const double L[7], const double R[7], double bnc, double gamma, double gammam1i, double F[7])
 {
   const double rol = L[0], vnl = L[1], vtl = L[2], vul = L[3], btl = L[4], bul = L[5], prl = L[6];
   const double ror = R[0], vnr = R[1], vtr = R[2], vur = R[3], btr = R[4], bur = R[5], prr = R[6];
   double gammam1 = gamma - 1.0;
   double gammam2 = gamma - 2.0;
-  double gammam1i = 1.0 / gammam1;
   double roli = 1.0 / rol;
   double rori = 1.0 / ror;
   double rrol = sqrt(rol);
@@ -1017,31 +1194,43 @@ QAS_HD void flux_roe(const double L[7], const double R[7], double bnc, double ga
                 ama * (-rvpaen) - a00 * rv00en);
 }
 
+QAS_HD void flux_roe(const double L[7], const double R[7], double bnc, double gamma, double F[7])
+{
+  flux_roe(L, R, bnc, gamma, 1.0 / (gamma - 1.0), F);
+}
+
+// gammam1i = 1/(gamma - 1), the same IEEE quotient wherever it is formed: the kernels take it from the host
+template <int RMN>
+QAS_HD void riemann(const double L[7], const double R[7], double bnc, double gamma, double gammam1i, double dv0,
+                                        double dv1, double F[7])
+{
+  if (RMN == 0)
+    flux_roe(L, R, bnc, gamma, gammam1i, F);
+  else if (RMN == 1)
+    flux_hlld<false>(L, R, bnc, gamma, gammam1i, dv0, dv1, F);
+  else if (RMN == 2)
+    flux_hlld<true>(L, R, bnc, gamma, gammam1i, dv0, dv1, F);
+  else
+    flux_mlau(L, R, bnc, gamma, gammam1i, dv0, dv1, F);
+}
 template <int RMN>
 QAS_HD void riemann(const double L[7], const double R[7], double bnc, double gamma, double dv0,
                                         double dv1, double F[7])
 {
-  if (RMN == 0)
-    flux_roe(L, R, bnc, gamma, F);
-  else if (RMN == 1)
-    flux_hlld<false>(L, R, bnc, gamma, dv0, dv1, F);
-  else if (RMN == 2)
-    flux_hlld<true>(L, R, bnc, gamma, dv0, dv1, F);
-  else
-    flux_mlau(L, R, bnc, gamma, dv0, dv1, F);
+  riemann<RMN>(L, R, bnc, gamma, 1.0 / (gamma - 1.0), dv0, dv1, F);
 }
 
 // the same flux handed to out(m, F[m]) as each component is final (MLAU emits while it runs;
 // the other solvers after their last component)
 template <int RMN, class Out>
-QAS_HD void riemann_out(const double L[7], const double R[7], double bnc, double gamma, double dv0, double dv1,
-                        Out &&out)
+QAS_HD void riemann_out(const double L[7], const double R[7], double bnc, double gamma, double gammam1i, double dv0,
+                        double dv1, Out &&out)
 {
   if constexpr (RMN == 3) {
-    flux_mlau_out(L, R, bnc, gamma, dv0, dv1, out);
+    flux_mlau_out(L, R, bnc, gamma, gammam1i, dv0, dv1, out);
   } else {
     double F[7];
-    riemann<RMN>(L, R, bnc, gamma, dv0, dv1, F);
+    riemann<RMN>(L, R, bnc, gamma, gammam1i, dv0, dv1, F);
 #pragma unroll
     for (int m = 0; m < 7; m++) out(m, F[m]);
   }

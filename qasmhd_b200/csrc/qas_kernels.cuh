@@ -48,6 +48,10 @@ namespace qas {
 
 constexpr int GH = 4;  // ghost cells per side
 
+constexpr int SWB = 128;  // threads of a face-sweep block
+constexpr int SLOTS = 9;  // states a face sweep hands on: ro, vn, vt, vu, bt, bu, pr, two induction states
+constexpr int SLP = 2 * SWB + 32;  // pitch of a slot: the block's right-face row(s), then its left-face rows
+
 struct Geo {
   int dim, nx, ny, nz;
   long long nd;
@@ -79,7 +83,7 @@ struct Maps {
 struct View {
   Geo g;
   int rmn, odr, rk, ctw;
-  double gam;
+  double gam, gm1i;  // gamma, 1/(gamma - 1)
   double dx, dy, dz;
   double *u[8];    // state ro,mx,my,mz,bx,by,bz,en
   double *u0[8];   // state at the start of the step (ut)
@@ -107,6 +111,17 @@ struct View {
 __device__ __forceinline__ long long cidx(const Geo &g, int i, int j, int k)
 {
   return (long long)g.nx * ((long long)g.ny * k + j) + i;
+}
+
+// element of an array by 32-bit byte offset (no array reaches 4 GB: the pool holds 77 of them): a base
+// from the kernel's parameters plus a 32-bit register needs no 64-bit address arithmetic
+__device__ __forceinline__ const double *at(const double *p, unsigned o)
+{
+  return reinterpret_cast<const double *>(reinterpret_cast<const char *>(p) + o);
+}
+__device__ __forceinline__ double *at(double *p, unsigned o)
+{
+  return reinterpret_cast<double *>(reinterpret_cast<char *>(p) + o);
 }
 
 __device__ __forceinline__ int map_src(const Maps &m, int G, int f, int a, int i)
@@ -281,10 +296,12 @@ __global__ void k_dv(View v)
 // ---------------------------------------------------------------------------
 // face states of each cell along axis A (mhd_lrstate + mhd_lr_fb)
 // ---------------------------------------------------------------------------
-// 6 resident blocks (80 registers, 52 B spilled to L1): 0.498 -> 0.478 ms per launch at KH 160^3,
-// unchanged in 2D; 5 blocks (96 registers) and 4 (118) are slower
+// Bound by FP64 issue (2 cycles a warp instruction) and, at 22 warps per SM, by the latency of a
+// block's first loads.  Per launch, OT 1024^2 x / KH 128^3 z: 104 / 268 us with 1096 FP64 operations
+// a cell and one copy of the interpolation per field, 7 blocks (72 registers) 88 / 228 us with 972
+// operations and the pair loop of face_states_emit; 6 blocks 91 / 243, 8 blocks 92 / 237.
 #ifndef QAS_LR_MINB
-#define QAS_LR_MINB 6
+#define QAS_LR_MINB 7
 #endif
 
 // stencil accessor of k_lr: field f of (ro, vn, vb, vc, cb, cc, pr) along axis A at point m
@@ -293,7 +310,11 @@ __global__ void k_dv(View v)
 template <int A>
 struct LrStencil {
   const View &v;
-  long long c, s;
+  unsigned c, s;  // byte offset of the cell, byte stride of the axis
+  __device__ __forceinline__ LrStencil(const View &v_, long long c_, long long s_)
+      : v(v_), c((unsigned)(8 * c_)), s((unsigned)(8 * s_))
+  {
+  }
   __device__ __forceinline__ const double *field(int f) const
   {
     constexpr int B = (A + 1) % 3, C = (A + 2) % 3;
@@ -307,9 +328,45 @@ struct LrStencil {
       default: return v.pr;
     }
   }
-  __device__ __forceinline__ double operator()(int f, int m) const { return __ldg(field(f) + c + (m - 2) * s); }
+  __device__ __forceinline__ double operator()(int f, int m) const { return __ldg(at(field(f), c + (m - 2) * s)); }
   // plain load, for reads issued after the face-state stores (kept in order behind them)
-  __device__ __forceinline__ double late(int f, int m) const { return field(f)[c + (m - 2) * s]; }
+  __device__ __forceinline__ double late(int f, int m) const { return *at(field(f), c + (m - 2) * s); }
+};
+
+// face_states of cell c along A by the reference's divisions, out of line: what the kernels call for
+// the rare cell whose smoothness leaves the range of the fast interpolation (they take the View as a
+// __grid_constant__ so that it is passed by address)
+template <int ODR, int A>
+__device__ __noinline__ void states_again(const View &v, long long c, double *l, double *r, long long ls)
+{
+  const LrStencil<A> st{v, c, v.g.s[A]};
+  double vl[7], vr[7];
+  face_states_of<ODR>(st, (A == 0 ? v.cx : (A == 1 ? v.cy : v.cz))[c], v.gam, vl, vr);
+  for (int m = 0; m < 7; m++) {
+    if (l) {
+      l[m * ls] = vl[m];
+      r[m * ls] = vr[m];
+    } else {
+      v.vl[m][c] = vl[m];
+      v.vr[m][c] = vr[m];
+    }
+  }
+}
+// the states of cell c into the face-state arrays
+template <int ODR, int A>
+struct StatesToHbm {
+  const View &v;
+  long long c;
+  __device__ __forceinline__ void operator()(int m, double l, double r) const
+  {
+    *at(v.vl[m], (unsigned)(8 * c)) = l;
+    *at(v.vr[m], (unsigned)(8 * c)) = r;
+  }
+  template <class ST>
+  __device__ __forceinline__ void again(const ST &, double, double) const
+  {
+    states_again<ODR, A>(v, c, nullptr, nullptr, 0);
+  }
 };
 
 // PR: the face-value form, 0 characteristic (mhd_m/a_reconst), 1 primitive (mhd_reconst), 2
@@ -319,17 +376,17 @@ struct LrStencil {
 template <int ODR, int A, int PR = -1, class ST>
 __device__ __forceinline__ void lr_cell(const View &v, long long c, long long s, const ST &st, double cnc)
 {
-  double vl[7], vr[7];
-  if (PR == 1 || (PR < 0 && v.recon == 1))
-    face_states_prim<ODR>(st, vl, vr);
-  else if (PR == 2 || (PR < 0 && v.recon == 2))
-    face_states_athena<ODR>(st, cnc, v.gam, vl, vr);
-  else
-    face_states_grouped<ODR>(st, cnc, v.gam, vl, vr);
+  const StatesToHbm<ODR, A> store{v, c};
+  if (PR == 1 || PR == 2 || (PR < 0 && v.recon != 0)) {
+    double vl[7], vr[7];
+    if (PR == 1 || (PR < 0 && v.recon == 1))
+      face_states_prim<ODR>(st, vl, vr);
+    else
+      face_states_athena<ODR>(st, cnc, v.gam, vl, vr);
 #pragma unroll
-  for (int m = 0; m < 7; m++) {
-    v.vl[m][c] = vl[m];
-    v.vr[m][c] = vr[m];
+    for (int m = 0; m < 7; m++) store(m, vl[m], vr[m]);
+  } else {
+    face_states_emit<ODR>(st, cnc, v.gam, store);
   }
   if (v.g.dim >= 2) {
     // the induction states are read after the face states are stored (keeps their loads from
@@ -370,7 +427,7 @@ __device__ __forceinline__ void lr_body(const View &v, int i, int j, int k)
   lr_cell<ODR, A, PR>(v, c, s, st, cn[c]);
 }
 template <int ODR, int A, int PR = 0>
-__global__ void __launch_bounds__(128, QAS_LR_MINB) k_lr(View v)
+__global__ void __launch_bounds__(128, QAS_LR_MINB) k_lr(const __grid_constant__ View v)
 {
   if (v.ctl->done) return;
   QAS_CELL_INDEX();
@@ -383,40 +440,64 @@ __global__ void __launch_bounds__(128, QAS_LR_MINB) k_lr(View v)
 // Stores one face's fluxes as the solver finishes them: F[0..3] to the mass and momentum fluxes
 // (normal component at 1+A), F[4] / F[5] minus the central part of the induction flux (also
 // stored, fc), F[6] plus the work of gravity.  The central parts come from the induction states
-// of the two cells: loaded here (LOADQ, the split form) or handed over in registers (fused).
-template <int A, bool LOADQ>
+// of the two cells, induction(t, l, r).
+template <int A, class Ind>
+__device__ __forceinline__ void store_flux(const View &v, long long f, long long s, int m, double x, double &f0,
+                                           Ind &&induction)
+{
+  constexpr int B = (A + 1) % 3, C = (A + 2) % 3;
+  const int dim = v.g.dim;
+  const unsigned o = (unsigned)(8 * f);
+  auto central = [&](int t) {
+    double l, r;
+    induction(t, l, r);
+    const double fc = 0.5 * (l + r);
+    *at(v.fc[A][t], o) = fc;
+    return fc;
+  };
+  if (m == 0) {
+    *at(v.f[A][0], o) = x;
+    f0 = x;
+  } else if (m == 1) {
+    *at(v.f[A][1 + A], o) = x;
+  } else if (m < 4) {
+    *at(v.f[A][1 + (m == 2 ? B : C)], o) = x;
+  } else if (m < 6) {
+    const int t = m - 4;
+    const bool ct = dim == 3 || (dim == 2 && A == t);  // a component of the CT update
+    *at(v.f[A][4 + (t == 0 ? B : C)], o) = ct ? x - central(t) : x;
+  } else {
+    // work done by gravity (2D/SERIAL/RTI/mhd2d_solve.cpp:197, :305; 3D/MPI/RTI/mhd3d_solve.cpp:247, :412, :577)
+    *at(v.f[A][7], o) = v.phi ? x + f0 * 0.5 * (v.phi[f - s] + v.phi[f]) : x;
+  }
+}
+// induction states in HBM (the split form)
+template <int A>
 struct FaceSink {
   const View &v;
   long long f, s;
-  double ql0, qr0, ql1, qr1;  // induction states when !LOADQ
   double f0;
-  __device__ __forceinline__ double central(int t)
-  {
-    const double l = LOADQ ? v.ql[t][f - s] : (t == 0 ? ql0 : ql1);
-    const double r = LOADQ ? v.qr[t][f] : (t == 0 ? qr0 : qr1);
-    const double fc = 0.5 * (l + r);
-    v.fc[A][t][f] = fc;
-    return fc;
-  }
   __device__ __forceinline__ void operator()(int m, double x)
   {
-    constexpr int B = (A + 1) % 3, C = (A + 2) % 3;
-    const int dim = v.g.dim;
-    switch (m) {
-      case 0:
-        v.f[A][0][f] = x;
-        f0 = x;
-        break;
-      case 1: v.f[A][1 + A][f] = x; break;
-      case 2: v.f[A][1 + B][f] = x; break;
-      case 3: v.f[A][1 + C][f] = x; break;
-      case 4: v.f[A][4 + B][f] = (dim == 3 || (dim == 2 && A == 0)) ? x - central(0) : x; break;
-      case 5: v.f[A][4 + C][f] = (dim == 3 || (dim == 2 && A == 1)) ? x - central(1) : x; break;
-      default:
-        // work done by gravity (2D/SERIAL/RTI/mhd2d_solve.cpp:197, :305; 3D/MPI/RTI/mhd3d_solve.cpp:247, :412, :577)
-        v.f[A][7][f] = v.phi ? x + f0 * 0.5 * (v.phi[f - s] + v.phi[f]) : x;
-        break;
-    }
+    store_flux<A>(v, f, s, m, x, f0, [&](int t, double &l, double &r) {
+      l = *at(v.ql[t], (unsigned)(8 * (f - s)));
+      r = *at(v.qr[t], (unsigned)(8 * f));
+    });
+  }
+};
+// induction states in a sweep's shared-memory slots
+template <int A>
+struct FaceSlots {
+  const View &v;
+  long long f, s;
+  const double *l, *r;
+  double f0;
+  __device__ __forceinline__ void operator()(int m, double x)
+  {
+    store_flux<A>(v, f, s, m, x, f0, [&](int t, double &ql, double &qr) {
+      ql = l[(7 + t) * SLP];
+      qr = r[(7 + t) * SLP];
+    });
   }
 };
 
@@ -433,11 +514,10 @@ __device__ __forceinline__ void flux_body(const View &v, int i, int j, int k)
   double L[7], R[7];
 #pragma unroll
   for (int m = 0; m < 7; m++) {
-    L[m] = v.vl[m][f - s];
-    R[m] = v.vr[m][f];
+    L[m] = *at(v.vl[m], (unsigned)(8 * (f - s)));
+    R[m] = *at(v.vr[m], (unsigned)(8 * f));
   }
-  const double bnf = v.u[4 + A][f];
-  const double bn = 0.5 * (bnf + bnf);
+  const double bn = v.u[4 + A][f];  // the reference's 0.5*(bn + bn)
   double dv0 = 0.0, dv1 = 0.0;
   if (RMN >= 2) {
     const double *vn = A == 0 ? v.vx : (A == 1 ? v.vy : v.vz);
@@ -450,7 +530,7 @@ __device__ __forceinline__ void flux_body(const View &v, int i, int j, int k)
       dv1 = qmin(qmin(d1[f - s], d1[f]), qmin(d2[f - s], d2[f]));
     }
   }
-  riemann_out<RMN>(L, R, bn, v.gam, dv0, dv1, FaceSink<A, true>{v, f, s, 0.0, 0.0, 0.0, 0.0, 0.0});
+  riemann_out<RMN>(L, R, bn, v.gam, v.gm1i, dv0, dv1, FaceSink<A>{v, f, s, 0.0});
 }
 // resident-block caps of the flux kernel per solver, measured on B200 per launch: Roe at 4
 // (128 registers, from 162) 0.0906 -> 0.0782 ms (KH 2D 1024^2); HLLD at 8 (64 registers, a
@@ -491,17 +571,24 @@ __global__ void __launch_bounds__(128, QAS_FLUX_MLAU_MINB) k_flux_mlau(View v)
 // the Riemann flux of every face in one kernel, so the face states never go
 // through HBM.
 //  * x faces: the cells pos in [2, nx-2) of all rows form one flattened
-//    sequence; warp w takes cells [31w, 31w+32) of it, and each lane hands its
-//    cell's right-face state to the next lane with a shuffle (31 faces per warp,
-//    every lane busy whatever the row length).
+//    sequence; warp w takes cells [31w, 31w+32) of it, and each lane reads its
+//    left neighbour's right-face state from that lane's shared-memory slots (31
+//    faces per warp, every lane busy whatever the row length).
 //  * y / z faces: one thread per column (x fastest, then the other transverse
 //    axis, flattened), marching along A over a segment of faces; the previous
-//    cell's right-face state waits in a shared-memory slot of the thread, not in
-//    registers, so the reconstruction and the Riemann solver do not hold it live.
-// Resident-block caps per Riemann solver: the reconstruction's 6 (80 registers),
-// Roe's 4 (its flux needs 128).  PR: 0 the characteristic or primitive reconstruction by
+//    cell's right-face state waits in the thread's other set of slots.
+// The reconstruction writes each component's two states to the thread's slots
+// as soon as they are final and the flux reads them from there, so neither
+// phase holds the other's values in registers.
+// The sweeps are bound by FP64 issue (55-60 % of the pipe), dependent FP64 latency and, along y / z,
+// by the latency of stencil loads.  Four warps on consecutive cells touch 8 planes a round where
+// four separate marches touch 20, so the planes stay in L1 (hit rate 28 -> 61 %); with slots instead of
+// registers, the pair loop and the prefetches, per launch at KH 128^3 (MLAU), x / y / z:
+// 388 / 435 / 427 -> 317 / 339 / 328 us.
+// Resident-block caps per Riemann solver: 6 (80 registers; 7 blocks 332 / 341 / 333, 5 blocks
+// 345 / 370 / 355 us), Roe's 4 (its flux needs 128; 5 blocks are slower).  PR: 0 the characteristic or primitive reconstruction by
 // v.recon (the default scheme), -1 also the Athena-type form, whose code raises the kernels'
-// register pressure (spills 156 -> 712 B).  Built for 4th-order interpolation (the other orders
+// register pressure (spills 200 -> 820 B).  Built for 4th-order interpolation (the other orders
 // take the two-kernel form).
 // ---------------------------------------------------------------------------
 #ifndef QAS_SWEEP_MINB
@@ -512,102 +599,117 @@ __global__ void __launch_bounds__(128, QAS_FLUX_MLAU_MINB) k_flux_mlau(View v)
 #endif
 #define QAS_SWEEP_MINB_OF(RMN) ((RMN) == 0 ? QAS_SWEEP_ROE_MINB : QAS_SWEEP_MINB)
 
+// the states of cell c into a thread's slots
+template <int ODR, int A>
+struct StatesToSlots {
+  const View &v;
+  long long c;
+  double *l, *r;
+  __device__ __forceinline__ void operator()(int m, double lv, double rv) const
+  {
+    l[m * SLP] = lv;
+    r[m * SLP] = rv;
+  }
+  template <class ST>
+  __device__ __forceinline__ void again(const ST &, double, double) const
+  {
+    states_again<ODR, A>(v, c, l, r, SLP);
+  }
+};
+
+// states of cell c: right face into the slots l[m * SLP], left face into r[m * SLP] (m < SLOTS).
 // PR: 0 the characteristic or primitive form by v.recon, -1 any of the three
 template <int ODR, int A, int PR>
-__device__ __forceinline__ void cell_states(const View &v, long long c, double vl[7], double vr[7], double ql[2],
-                                            double qr[2])
+__device__ __forceinline__ void cell_states(const View &v, long long c, double *l, double *r)
 {
   const Geo &g = v.g;
   const long long s = g.s[A];
-  constexpr int B = (A + 1) % 3, C = (A + 2) % 3;
-  const double *vn = A == 0 ? v.vx : (A == 1 ? v.vy : v.vz);
-  const double *vb = B == 0 ? v.vx : (B == 1 ? v.vy : v.vz);
-  const double *vc = C == 0 ? v.vx : (C == 1 ? v.vy : v.vz);
   const double *cn = A == 0 ? v.cx : (A == 1 ? v.cy : v.cz);
-  const double *cb = B == 0 ? v.cx : (B == 1 ? v.cy : v.cz);
-  const double *ccp = C == 0 ? v.cx : (C == 1 ? v.cy : v.cz);
   const LrStencil<A> st{v, c, s};
-  if (PR <= 0 && v.recon == 1)
-    face_states_prim<ODR>(st, vl, vr);
-  else if (PR < 0 && v.recon == 2)
-    face_states_athena<ODR>(st, __ldg(cn + c), v.gam, vl, vr);
-  else
-    face_states_grouped<ODR>(st, __ldg(cn + c), v.gam, vl, vr);
+  const StatesToSlots<ODR, A> store{v, c, l, r};
+  if ((PR <= 0 && v.recon == 1) || (PR < 0 && v.recon == 2)) {
+    double vl[7], vr[7];
+    if (PR < 0 && v.recon == 2)
+      face_states_athena<ODR>(st, __ldg(at(cn, st.c)), v.gam, vl, vr);
+    else
+      face_states_prim<ODR>(st, vl, vr);
+#pragma unroll
+    for (int m = 0; m < 7; m++) store(m, vl[m], vr[m]);
+  } else {
+    face_states_emit<ODR>(st, __ldg(at(cn, st.c)), v.gam, store);
+  }
   if (g.dim >= 2) {
-    const double *bnf = v.u[4 + A];
-    const double bfl = __ldg(bnf + c + s), bfr = __ldg(bnf + c);
+    const double bfl = __ldg(at(v.u[4 + A], st.c + st.s)), bfr = __ldg(at(v.u[4 + A], st.c));
 #pragma unroll
     for (int t = 0; t < 2; t++) {
       if (g.dim == 2 && ((A == 0 && t == 1) || (A == 1 && t == 0))) continue;
-      const double *vt = t == 0 ? vb : vc;
-      const double *bt = t == 0 ? cb : ccp;
       double prod[5], vts[5];
 #pragma unroll
       for (int m = 0; m < 5; m++) {
-        const long long p = c + (m - 2) * s;
-        prod[m] = __ldg(bt + p) * __ldg(vn + p);
-        vts[m] = __ldg(vt + p);
+        prod[m] = st(4 + t, m) * st(1, m);  // bt * vn
+        vts[m] = st(2 + t, m);              // vt
       }
       double fl0, fr0, fl1, fr1;
       lin_lr<ODR>(prod, fl0, fr0);
       lin_lr<ODR>(vts, fl1, fr1);
-      ql[t] = fl0 - bfl * fl1;
-      qr[t] = fr0 - bfr * fr1;
+      store(7 + t, fl0 - bfl * fl1, fr0 - bfr * fr1);
     }
   }
 }
 
-// flux at face f from the left cell's right-face state L/QL and this cell's left-face state R/QR
+// flux at face f from the left cell's right-face state, slots l[m * SLP], and this cell's left-face
+// state, slots r[m * SLP]
 template <int RMN, int A>
-__device__ __forceinline__ void face_flux(const View &v, long long f, const double L[7], const double R[7],
-                                          const double QL[2], const double QR[2])
+__device__ __forceinline__ void face_flux(const View &v, long long f, const double *l, const double *r)
 {
   const Geo &g = v.g;
   const long long s = g.s[A];
   constexpr int B = (A + 1) % 3, C = (A + 2) % 3;
-  const double bnf = __ldg(v.u[4 + A] + f);
-  const double bn = 0.5 * (bnf + bnf);
+  const unsigned o = (unsigned)(8 * f), so = (unsigned)(8 * s);
+  const double bn = __ldg(at(v.u[4 + A], o));  // the reference's 0.5*(bn + bn)
   double dv0 = 0.0, dv1 = 0.0;
   if (RMN >= 2) {
     const double *vn = A == 0 ? v.vx : (A == 1 ? v.vy : v.vz);
-    dv0 = __ldg(vn + f) - __ldg(vn + f - s);
+    dv0 = __ldg(at(vn, o)) - __ldg(at(vn, o - so));
     if (g.dim == 2) {
       const double *dt = v.dv[A == 0 ? 1 : 0];
-      dv1 = qmin(__ldg(dt + f - s), __ldg(dt + f));
+      dv1 = qmin(__ldg(at(dt, o - so)), __ldg(at(dt, o)));
     } else if (g.dim == 3) {
       const double *d1 = v.dv[B], *d2 = v.dv[C];
-      dv1 = qmin(qmin(__ldg(d1 + f - s), __ldg(d1 + f)), qmin(__ldg(d2 + f - s), __ldg(d2 + f)));
+      dv1 = qmin(qmin(__ldg(at(d1, o - so)), __ldg(at(d1, o))), qmin(__ldg(at(d2, o - so)), __ldg(at(d2, o))));
     }
   }
-  riemann_out<RMN>(L, R, bn, v.gam, dv0, dv1, FaceSink<A, false>{v, f, s, QL[0], QR[0], QL[1], QR[1], 0.0});
+  double L[7], R[7];
+#pragma unroll
+  for (int m = 0; m < 7; m++) {
+    L[m] = l[m * SLP];
+    R[m] = r[m * SLP];
+  }
+  riemann_out<RMN>(L, R, bn, v.gam, v.gm1i, dv0, dv1, FaceSlots<A>{v, f, s, l, r, 0.0});
 }
 
 // one lane of an x-sweep warp: the face states of cell (i, j, k) (a valid cell even for a lane
-// past the end, have_cell false, so that the warp stays converged), the hand-off of the right-face
-// state to the next lane, and the flux at the cell's left face when the previous lane holds the
-// cell to its left (i >= 3)
+// past the end, have_cell false, so that the warp stays converged) and the flux at the cell's
+// left face when the previous lane holds the cell to its left (i >= 3)
 template <int ODR, int RMN, int PR>
-__device__ __forceinline__ void sweep_x_cell(const View &v, int i, int j, int k, int lane, bool have_cell)
+__device__ __forceinline__ void sweep_x_cell(const View &v, int i, int j, int k, int lane, bool have_cell, double *sm)
 {
   const long long c = cidx(v.g, i, j, k);
-  double vl[7], vr[7], ql[2] = {0.0, 0.0}, qr[2] = {0.0, 0.0};
-  cell_states<ODR, 0, PR>(v, c, vl, vr, ql, qr);
-  double L[7], QL[2];
-#pragma unroll
-  for (int m = 0; m < 7; m++) L[m] = __shfl_up_sync(0xffffffffu, vl[m], 1);
-  QL[0] = __shfl_up_sync(0xffffffffu, ql[0], 1);
-  QL[1] = __shfl_up_sync(0xffffffffu, ql[1], 1);
-  if (lane >= 1 && have_cell && i >= 3) face_flux<RMN, 0>(v, c, L, vr, QL, qr);
+  double *l = sm + threadIdx.x, *r = l + SWB;
+  cell_states<ODR, 0, PR>(v, c, l, r);
+  __syncwarp();
+  if (lane >= 1 && have_cell && i >= 3) face_flux<RMN, 0>(v, c, l - 1, r);
 }
 
-// x sweep: 4 warps per block, 31 faces per warp over the flattened cells of all rows
+// x sweep: 31 faces per warp over the flattened cells of all rows
 template <int ODR, int RMN, int PR>
-__global__ void __launch_bounds__(128, QAS_SWEEP_MINB_OF(RMN)) k_sweep_x(View v, long long nwarps)
+__global__ void __launch_bounds__(SWB, QAS_SWEEP_MINB_OF(RMN)) k_sweep_x(const __grid_constant__ View v, long long nwarps)
 {
   if (v.ctl->done) return;
+  __shared__ double sm[SLOTS * SLP];
   const Geo &g = v.g;
   const int lane = threadIdx.x & 31;
-  const long long w = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+  const long long w = (long long)blockIdx.x * (SWB / 32) + (threadIdx.x >> 5);
   if (w >= nwarps) return;  // the whole warp leaves together
   const long long ncell = g.nx - 4;
   const long long total = ncell * g.ny * g.nz;
@@ -616,93 +718,66 @@ __global__ void __launch_bounds__(128, QAS_SWEEP_MINB_OF(RMN)) k_sweep_x(View v,
   if (!have_cell) t = total - 1;  // a valid cell, computed and discarded (keeps the warp converged)
   const long long row = t / ncell;
   const int i = 2 + (int)(t - row * ncell);
-  const long long c = cidx(g, i, (int)(row % g.ny), (int)(row / g.ny));
-  double vl[7], vr[7], ql[2] = {0.0, 0.0}, qr[2] = {0.0, 0.0};
-  cell_states<ODR, 0, PR>(v, c, vl, vr, ql, qr);
-  double L[7], QL[2];
-#pragma unroll
-  for (int m = 0; m < 7; m++) L[m] = __shfl_up_sync(0xffffffffu, vl[m], 1);
-  QL[0] = __shfl_up_sync(0xffffffffu, ql[0], 1);
-  QL[1] = __shfl_up_sync(0xffffffffu, ql[1], 1);
-  // lane-1 holds cell i-1 of the same row exactly when i >= 3
-  if (lane >= 1 && have_cell && i >= 3) face_flux<RMN, 0>(v, c, L, vr, QL, qr);
+  sweep_x_cell<ODR, RMN, PR>(v, i, (int)(row % g.ny), (int)(row / g.ny), lane, have_cell, sm);
 }
 
-// one column of a y / z sweep: the faces p in [p0, p1) along A of the column through (i, o)
-// (o = k for the y sweep, j for the z sweep), from the cell before p0 on; the previous cell's
-// right-face state waits in the thread's shared-memory slot carry[.][tid]
+__device__ __forceinline__ void prefetch_l1(const double *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
+// one block's 32 columns of a y / z sweep: the faces p in [p0, p1) along A of the columns through
+// (i, o) (o = k for the y sweep, j for the z sweep; `have`: this lane has a column), from the cell
+// before p0 on.  The block's warps take consecutive cells, so that they share their stencils' lines
+// in L1; warp w's cell is handed to warp w + 1 through row w + 1 of the slots, the last warp's
+// to the next round through row 0.
 template <int ODR, int RMN, int A, int PR>
-__device__ __forceinline__ void sweep_column(const View &v, int i, int o, int p0, int p1, double (*carry)[128], int tid)
+__device__ __forceinline__ void sweep_columns(const View &v, int i, int o, bool have, int p0, int p1, double *sm)
 {
-  const Geo &g = v.g;
-  const long long s = g.s[A];
-  long long c = A == 1 ? cidx(g, i, p0 - 1, o) : cidx(g, i, o, p0 - 1);
-  {
-    double vl[7], vr[7], ql[2] = {0.0, 0.0}, qr[2] = {0.0, 0.0};
-    cell_states<ODR, A, PR>(v, c, vl, vr, ql, qr);
+  constexpr int NW = SWB / 32;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double *l = sm + 32 * w + lane, *r = sm + 32 * (NW + 1) + 32 * w + lane;
+  const long long s = v.g.s[A];
+  const int first = p0 - 1;
+  long long c = A == 1 ? cidx(v.g, i, first + w, o) : cidx(v.g, i, o, first + w);
+#pragma unroll 1
+  for (int p = first; p < p1; p += NW) {
+    const bool cell = have && p + w < p1;
+    if (p > first && w == NW - 1) {
 #pragma unroll
-    for (int m = 0; m < 7; m++) carry[m][tid] = vl[m];
-    carry[7][tid] = ql[0];
-    carry[8][tid] = ql[1];
-  }
-  for (int p = p0; p < p1; p++) {
-    c += s;
-    double vl[7], vr[7], ql[2] = {0.0, 0.0}, qr[2] = {0.0, 0.0};
-    cell_states<ODR, A, PR>(v, c, vl, vr, ql, qr);
-    double L[7], QL[2];
-#pragma unroll
-    for (int m = 0; m < 7; m++) {
-      L[m] = carry[m][tid];
-      carry[m][tid] = vl[m];
+      for (int m = 0; m < SLOTS; m++) l[m * SLP - 32 * (NW - 1)] = l[m * SLP + 32];
     }
-    QL[0] = carry[7][tid];
-    QL[1] = carry[8][tid];
-    carry[7][tid] = ql[0];
-    carry[8][tid] = ql[1];
-    face_flux<RMN, A>(v, c, L, vr, QL, qr);
+    if (cell && RMN >= 2) {  // what the flux reads besides the states
+      constexpr int B = (A + 1) % 3, C = (A + 2) % 3;
+      prefetch_l1(v.dv[B] + c);
+      prefetch_l1(v.dv[C] + c);
+      prefetch_l1(v.u[4 + A] + c);
+    }
+    if (cell) cell_states<ODR, A, PR>(v, c, l + 32, r);
+    if (have && p + NW + w < p1) {  // the plane that this warp's next stencil adds
+      const long long q = c + (NW + 2) * s;
+      const LrStencil<A> st{v, c, s};
+#pragma unroll
+      for (int f = 0; f < 7; f++) prefetch_l1(at(st.field(f), (unsigned)(8 * q)));
+    }
+    __syncthreads();
+    if (cell && p + w >= p0) face_flux<RMN, A>(v, c, l, r);
+    __syncthreads();
+    c += NW * s;
   }
 }
 
-// y / z sweep: one thread per column, marching over `seg` faces along A
+// y / z sweep: 32 columns per block, marching over `seg` faces along A
 template <int ODR, int RMN, int A, int PR>
-__global__ void __launch_bounds__(128, QAS_SWEEP_MINB_OF(RMN)) k_sweep_m(View v, int seg)
+__global__ void __launch_bounds__(SWB, QAS_SWEEP_MINB_OF(RMN)) k_sweep_m(const __grid_constant__ View v, int seg)
 {
   if (v.ctl->done) return;
   const Geo &g = v.g;
-  __shared__ double carry[9][128];  // previous cell's right-face state and induction state, per thread
-  const int tid = threadIdx.x;
+  __shared__ double sm[SLOTS * SLP];
   const int no = A == 1 ? g.nz : g.ny;  // extent of the other transverse axis
-  const long long col = (long long)blockIdx.x * 128 + tid;
-  if (col >= (long long)g.nx * no) return;  // no barrier below: threads leave freely
-  const int i = (int)(col % g.nx), o = (int)(col / g.nx);
+  const long long cols = (long long)g.nx * no;
+  long long col = (long long)blockIdx.x * 32 + (threadIdx.x & 31);
+  const bool have = col < cols;
+  if (!have) col = cols - 1;
   const int p0 = 3 + blockIdx.y * seg;
-  const int p1 = min(p0 + seg, g.n[A] - 2);
-  const long long s = g.s[A];
-  long long c = A == 1 ? cidx(g, i, p0 - 1, o) : cidx(g, i, o, p0 - 1);
-  {
-    double vl[7], vr[7], ql[2] = {0.0, 0.0}, qr[2] = {0.0, 0.0};
-    cell_states<ODR, A, PR>(v, c, vl, vr, ql, qr);
-#pragma unroll
-    for (int m = 0; m < 7; m++) carry[m][tid] = vl[m];
-    carry[7][tid] = ql[0];
-    carry[8][tid] = ql[1];
-  }
-  for (int p = p0; p < p1; p++) {
-    c += s;
-    double vl[7], vr[7], ql[2] = {0.0, 0.0}, qr[2] = {0.0, 0.0};
-    cell_states<ODR, A, PR>(v, c, vl, vr, ql, qr);
-    double L[7], QL[2];
-#pragma unroll
-    for (int m = 0; m < 7; m++) {
-      L[m] = carry[m][tid];
-      carry[m][tid] = vl[m];
-    }
-    QL[0] = carry[7][tid];
-    QL[1] = carry[8][tid];
-    carry[7][tid] = ql[0];
-    carry[8][tid] = ql[1];
-    face_flux<RMN, A>(v, c, L, vr, QL, qr);
-  }
+  sweep_columns<ODR, RMN, A, PR>(v, (int)(col % g.nx), (int)(col / g.nx), have, p0, min(p0 + seg, g.n[A] - 2), sm);
 }
 
 // ---------------------------------------------------------------------------

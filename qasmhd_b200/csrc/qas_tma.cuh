@@ -130,7 +130,7 @@ struct LrTmaShape {
 };
 
 template <int ODR, int A, int TX, int TR, int MA>
-__global__ void __launch_bounds__(TX *TR, 5) k_lr_tma(View v, const __grid_constant__ LrTmaMaps maps, LrTmaPlan pl)
+__global__ void __launch_bounds__(TX *TR, 5) k_lr_tma(const __grid_constant__ View v, const __grid_constant__ LrTmaMaps maps, LrTmaPlan pl)
 {
   using S = LrTmaShape<A, TX, TR>;
   constexpr int NF = 7;

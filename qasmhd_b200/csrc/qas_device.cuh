@@ -89,6 +89,23 @@ QAS_HD double flip(double x, bool neg)
 #endif
 }
 
+// x/24 rounded to nearest by two operations instead of a division: with h + l = 1/24 to 106
+// bits, x*h + RN(x*l) is within 2^-50 ulp of x/24, and no x/24 lies nearer than 1/6 ulp to a
+// rounding boundary (24 = 3*8; Brisebarre, Muller, Raina, IEEE Trans. Comput. 53, 2004, division
+// by a constant).  Below 2^-900, where x*l would lose bits, the division itself.
+QAS_HD double div24(double x)
+{
+#if defined(__CUDA_ARCH__)
+  const double h = 1.0 / 24.0;                  // RN(1/24) = (1 - 2^-54)/24: 24 h = 1 - 2^-54
+  const double l = 5.5511151231257827e-17 / 24.0;  // (1 - 24 h)/24, 2^-54/24
+  const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  if (hi < 0x07b00000u && (hi | (unsigned)__double2loint(x)) != 0u) return x / 24.0;  // tiny, not zero
+  return fma(x, h, x * l);
+#else
+  return x / 24.0;
+#endif
+}
+
 QAS_HD double qmax(double a, double b) { return (a >= b) ? a : b; }
 QAS_HD double qmin(double a, double b) { return (a >= b) ? b : a; }
 QAS_HD double minmod(double a, double b)
@@ -109,7 +126,7 @@ QAS_HD double fcen(double fm, double f0, double f1, double f2)
 template <int ODR>
 QAS_HD double dfc(double fm, double f0, double f1, double f2)
 {
-  if (ODR >= 3) return ((27.0 * (f1 - f0) - (f2 - fm)) / 24.0);
+  if (ODR >= 3) return div24(27.0 * (f1 - f0) - (f2 - fm));
   return (f1 - f0);
 }
 

@@ -1,5 +1,6 @@
-// The short reciprocal of qas_device.cuh against the compiler's IEEE division, bit for bit, on the
-// device: rcp_normal(x) == 1.0/x.  Prints the number of differing inputs and exits 1 if there are any.
+// The short division forms of qas_device.cuh against the compiler's IEEE divisions, bit for bit, on
+// the device: rcp_normal(x) == 1.0/x and div24(x) == x/24.  Prints the number of differing inputs
+// per set and exits 1 if there are any.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -43,14 +44,34 @@ __global__ void k_rcp(unsigned long long n, unsigned long long seed, unsigned lo
     if (!same(rcp_normal(x), 1.0 / x)) atomicAdd(bad, 1ull);
   }
 }
+// every exponent, zeros, subnormals, infinities and NaN among them; multiples of 24 and of 12
+__global__ void k_div24(unsigned long long n, unsigned long long seed, unsigned long long *bad)
+{
+  for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
+       i += (unsigned long long)gridDim.x * blockDim.x) {
+    const unsigned long long r = mix(i + seed), q = mix(r);
+    double x;
+    switch (q & 7) {
+      case 0: x = (double)(long long)(r >> 16) * 24.0; break;
+      case 1: x = (double)(long long)(r >> 16) * 12.0; break;
+      case 2: x = from_bits((q >> 3) & 1, (q >> 20) % 8, r >> ((q >> 32) % 52)); break;
+      case 3: x = from_bits((q >> 3) & 1, 100 + (q >> 20) % 60, r); break;
+      case 4: x = from_bits((q >> 3) & 1, 2040 + (q >> 20) % 8, r & ((q >> 31) & 1 ? ~0ull : 0ull)); break;
+      default: x = from_bits((q >> 3) & 1, (q >> 20) % 2048, r); break;
+    }
+    if (!same(div24(x), x / 24.0)) atomicAdd(bad, 1ull);
+  }
+}
+
 int main(int argc, char **argv)
 {
   const unsigned long long n = argc > 1 ? strtoull(argv[1], nullptr, 10) : 1ull << 28;
-  unsigned long long *bad, h[1] = {0};
+  unsigned long long *bad, h[2] = {0, 0};
   if (cudaMalloc(&bad, sizeof(h)) != cudaSuccess || cudaMemset(bad, 0, sizeof(h)) != cudaSuccess) return 2;
   k_rcp<<<1184, 256>>>(n, 1, &bad[0]);
+  k_div24<<<1184, 256>>>(n, 2, &bad[1]);
   if (cudaMemcpy(h, bad, sizeof(h), cudaMemcpyDeviceToHost) != cudaSuccess) return 2;
-  printf("rcp_normal %llu differing of %llu\n", h[0], n);
+  printf("rcp_normal %llu div24 %llu differing of %llu\n", h[0], h[1], n);
   cudaFree(bad);
-  return h[0] ? 1 : 0;
+  return h[0] || h[1] ? 1 : 0;
 }

@@ -185,18 +185,6 @@ __global__ void kb_bound(const View *__restrict__ views, BMap map)
   QAS_BATCH_END
 }
 
-// u0 = u for all cells of every instance (the copy of ut at the start of ideal)
-__global__ void kb_copy_u0(const View *__restrict__ views, BMap map)
-{
-  QAS_BATCH_BLOCKS(map)
-  if (QAS_BATCH_CELL_OK) {
-    const long long c = cidx(v.g, ti, tj, tk);
-#pragma unroll
-    for (int m = 0; m < 8; m++) v.u0[m][c] = v.u[m][c];
-  }
-  QAS_BATCH_END
-}
-
 // per-instance control: one thread per instance
 __global__ void kb_begin(const View *__restrict__ views, int n, int check_tim)
 {

@@ -189,7 +189,7 @@ __global__ void QAS_EMF_BOUNDS kw_emf(View v, Rows2 r)
 // the update cells of k_update (i in [GH, nx-GH], likewise j in 3D) on planes [lo, hi), which
 // lie in [GH, n-GH] (the last face plane of the staggered field included)
 template <int ODR>
-__global__ void QAS_UPDATE_BOUNDS kw_update(View v, Rows2 r, double c0, double c1, StatePtrs src)
+__global__ void QAS_UPDATE_BOUNDS kw_update(View v, Rows2 r, double c0, double c1)
 {
   QAS_PDL_WAIT();
   if (v.ctl->done) return;
@@ -208,7 +208,7 @@ __global__ void QAS_UPDATE_BOUNDS kw_update(View v, Rows2 r, double c0, double c
     if (tk > 0 || j < 0) return;
   }
   if (i > g.nx - GH) return;
-  update_body<ODR>(v, i, j, k, c0, c1, src.p);  // U_r of the cell from U_{r-1} (src) and ut
+  update_body<ODR>(v, i, j, k, c0, c1);  // U_r (v.uo) of the cell from U_{r-1} (v.u) and ut
 }
 
 // ghost fill of the cells of planes [lo, hi) that are ghosts along an in-plane axis (x in 2D;

@@ -309,6 +309,39 @@ void prof_mark(qas_ctx *c, int kid)
 }
 void prof_done(qas_ctx *c) { cudaEventRecord(c->prof_events[2 * (c->prof_kids.size() - 1) + 1], c->stream); }
 
+template <typename... KArgs, typename... Args>
+long long pdl_launch(cudaError_t &err, void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args)
+{
+  if (grid.x == 0 || grid.y == 0 || grid.z == 0) return 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = 0;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+  if (e != cudaSuccess && err == cudaSuccess) err = e;
+  return 1;
+}
+
+// one kernel on the context's stream; issued eagerly with programmatic stream serialization, which hides
+// the launch latency behind the kernel before (OT 128x96: 389 -> 267 us for two steps of single calls),
+// in a graph with plain edges, which are the faster ones there (OT 200^2: 150 against 165 us a step).
+// Only kernels that begin with pdl_begin().  An error stays with the runtime (check_launch)
+template <class... KArgs, class... Args>
+void launch(qas_ctx *c, void (*kern)(KArgs...), dim3 grid, dim3 block, Args... args)
+{
+  cudaError_t e = cudaSuccess;
+  if (c->capturing)
+    kern<<<grid, block, 0, c->stream>>>(args...);
+  else
+    pdl_launch(e, kern, grid, block, c->stream, args...);
+}
+
 // launch `expr` (one kernel) with optional event timing
 #define QL(c, kid, ...)                    \
   do {                                     \
@@ -477,33 +510,33 @@ void launch_lr(qas_ctx *c, int a)
   }
   const dim3 grid = cells_grid(c->geo, c->tile[KID_LR]), blk = c->tile[KID_LR];
   if (c->view.recon == 1) {
-    if (a == 0) QL(c, KID_LR, k_lr<ODR, 0, 1><<<grid, blk, 0, c->stream>>>(c->view));
-    if (a == 1) QL(c, KID_LR, k_lr<ODR, 1, 1><<<grid, blk, 0, c->stream>>>(c->view));
-    if (a == 2) QL(c, KID_LR, k_lr<ODR, 2, 1><<<grid, blk, 0, c->stream>>>(c->view));
+    if (a == 0) QL(c, KID_LR, launch(c, k_lr<ODR, 0, 1>, grid, blk, c->view));
+    if (a == 1) QL(c, KID_LR, launch(c, k_lr<ODR, 1, 1>, grid, blk, c->view));
+    if (a == 2) QL(c, KID_LR, launch(c, k_lr<ODR, 2, 1>, grid, blk, c->view));
     return;
   }
   if (c->view.recon == 2) {
-    if (a == 0) QL(c, KID_LR, k_lr<ODR, 0, 2><<<grid, blk, 0, c->stream>>>(c->view));
-    if (a == 1) QL(c, KID_LR, k_lr<ODR, 1, 2><<<grid, blk, 0, c->stream>>>(c->view));
-    if (a == 2) QL(c, KID_LR, k_lr<ODR, 2, 2><<<grid, blk, 0, c->stream>>>(c->view));
+    if (a == 0) QL(c, KID_LR, launch(c, k_lr<ODR, 0, 2>, grid, blk, c->view));
+    if (a == 1) QL(c, KID_LR, launch(c, k_lr<ODR, 1, 2>, grid, blk, c->view));
+    if (a == 2) QL(c, KID_LR, launch(c, k_lr<ODR, 2, 2>, grid, blk, c->view));
     return;
   }
-  if (a == 0) QL(c, KID_LR, k_lr<ODR, 0><<<grid, blk, 0, c->stream>>>(c->view));
-  if (a == 1) QL(c, KID_LR, k_lr<ODR, 1><<<grid, blk, 0, c->stream>>>(c->view));
-  if (a == 2) QL(c, KID_LR, k_lr<ODR, 2><<<grid, blk, 0, c->stream>>>(c->view));
+  if (a == 0) QL(c, KID_LR, launch(c, k_lr<ODR, 0>, grid, blk, c->view));
+  if (a == 1) QL(c, KID_LR, launch(c, k_lr<ODR, 1>, grid, blk, c->view));
+  if (a == 2) QL(c, KID_LR, launch(c, k_lr<ODR, 2>, grid, blk, c->view));
 }
 template <int RMN>
 void launch_flux(qas_ctx *c, int a)
 {
   if constexpr (RMN == 3) {
-    if (a == 0) QL(c, KID_FLUX, k_flux_mlau<0><<<cells_grid(c->geo, c->tile[KID_FLUX]), c->tile[KID_FLUX], 0, c->stream>>>(c->view));
-    if (a == 1) QL(c, KID_FLUX, k_flux_mlau<1><<<cells_grid(c->geo, c->tile[KID_FLUX]), c->tile[KID_FLUX], 0, c->stream>>>(c->view));
-    if (a == 2) QL(c, KID_FLUX, k_flux_mlau<2><<<cells_grid(c->geo, c->tile[KID_FLUX]), c->tile[KID_FLUX], 0, c->stream>>>(c->view));
+    if (a == 0) QL(c, KID_FLUX, launch(c, k_flux_mlau<0>, cells_grid(c->geo, c->tile[KID_FLUX]), c->tile[KID_FLUX], c->view));
+    if (a == 1) QL(c, KID_FLUX, launch(c, k_flux_mlau<1>, cells_grid(c->geo, c->tile[KID_FLUX]), c->tile[KID_FLUX], c->view));
+    if (a == 2) QL(c, KID_FLUX, launch(c, k_flux_mlau<2>, cells_grid(c->geo, c->tile[KID_FLUX]), c->tile[KID_FLUX], c->view));
     return;
   } else {
-    if (a == 0) QL(c, KID_FLUX, k_flux<RMN, 0><<<cells_grid(c->geo, c->tile[KID_FLUX]), c->tile[KID_FLUX], 0, c->stream>>>(c->view));
-    if (a == 1) QL(c, KID_FLUX, k_flux<RMN, 1><<<cells_grid(c->geo, c->tile[KID_FLUX]), c->tile[KID_FLUX], 0, c->stream>>>(c->view));
-    if (a == 2) QL(c, KID_FLUX, k_flux<RMN, 2><<<cells_grid(c->geo, c->tile[KID_FLUX]), c->tile[KID_FLUX], 0, c->stream>>>(c->view));
+    if (a == 0) QL(c, KID_FLUX, launch(c, k_flux<RMN, 0>, cells_grid(c->geo, c->tile[KID_FLUX]), c->tile[KID_FLUX], c->view));
+    if (a == 1) QL(c, KID_FLUX, launch(c, k_flux<RMN, 1>, cells_grid(c->geo, c->tile[KID_FLUX]), c->tile[KID_FLUX], c->view));
+    if (a == 2) QL(c, KID_FLUX, launch(c, k_flux<RMN, 2>, cells_grid(c->geo, c->tile[KID_FLUX]), c->tile[KID_FLUX], c->view));
   }
 }
 
@@ -579,17 +612,17 @@ void launch_sweep_pr(qas_ctx *c, int a)
     const long long total = (long long)(g.nx - 4) * g.ny * g.nz;
     const long long nwarps = (total - 2) / 31 + 1;
     const unsigned nb = (unsigned)((nwarps + SWB / 32 - 1) / (SWB / 32));
-    QL(c, KID_SWEEP, k_sweep_x<4, RMN, PR><<<nb, SWB, 0, c->stream>>>(c->view, nwarps));
+    QL(c, KID_SWEEP, launch(c, k_sweep_x<4, RMN, PR>, nb, SWB, c->view, nwarps));
     return;
   }
   const unsigned colb = (unsigned)(((long long)g.nx * (a == 1 ? g.nz : g.ny) + 31) / 32);
   const int len = g.n[a] - 5;
   if (a == 1) {
     const int seg = sweep_seg(c, 1, (const void *)k_sweep_m<4, RMN, 1, 0>);
-    QL(c, KID_SWEEP, k_sweep_m<4, RMN, 1, PR><<<dim3(colb, (len + seg - 1) / seg), SWB, 0, c->stream>>>(c->view, seg));
+    QL(c, KID_SWEEP, launch(c, k_sweep_m<4, RMN, 1, PR>, dim3(colb, (len + seg - 1) / seg), SWB, c->view, seg));
   } else {
     const int seg = sweep_seg(c, 2, (const void *)k_sweep_m<4, RMN, 2, 0>);
-    QL(c, KID_SWEEP, k_sweep_m<4, RMN, 2, PR><<<dim3(colb, (len + seg - 1) / seg), SWB, 0, c->stream>>>(c->view, seg));
+    QL(c, KID_SWEEP, launch(c, k_sweep_m<4, RMN, 2, PR>, dim3(colb, (len + seg - 1) / seg), SWB, c->view, seg));
   }
 }
 template <int RMN>
@@ -636,14 +669,14 @@ long long launch_crcte(qas_ctx *c)
 template <int ODR>
 long long stage_prim(qas_ctx *c)
 {
-  QL(c, KID_PRIM, k_prim<ODR><<<cells_grid(c->geo, c->tile[KID_PRIM]), c->tile[KID_PRIM], 0, c->stream>>>(c->view));
+  QL(c, KID_PRIM, launch(c, k_prim<ODR>, cells_grid(c->geo, c->tile[KID_PRIM]), c->tile[KID_PRIM], c->view));
   return 1;
 }
 bool stage_has_dv(const qas_ctx *c) { return c->scheme.rmn >= 2 && c->geo.dim >= 2; }
 long long stage_dv(qas_ctx *c)
 {
   if (!stage_has_dv(c)) return 0;
-  QL(c, KID_DV, k_dv<<<cells_grid(c->geo, c->tile[KID_DV]), c->tile[KID_DV], 0, c->stream>>>(c->view));
+  QL(c, KID_DV, launch(c, k_dv, cells_grid(c->geo, c->tile[KID_DV]), c->tile[KID_DV], c->view));
   return 1;
 }
 template <int ODR>
@@ -676,13 +709,13 @@ long long stage_rest(qas_ctx *c, double c0, double c1)
   }
   nk += launch_crcte(c);  // 1D Hall driver with electron inertia (hmhd1d_solve.cpp:98-108)
   if (g.dim >= 2) {
-    QL(c, KID_EMF, k_emf<ODR><<<cells_grid(g, c->tile[KID_EMF]), c->tile[KID_EMF], 0, c->stream>>>(c->view));
+    QL(c, KID_EMF, launch(c, k_emf<ODR>, cells_grid(g, c->tile[KID_EMF]), c->tile[KID_EMF], c->view));
     nk++;
   }
-  QL(c, KID_UPDATE, k_update<ODR><<<update_grid(g, c->tile[KID_UPDATE]), c->tile[KID_UPDATE], 0, c->stream>>>(c->view, c0, c1));
+  QL(c, KID_UPDATE, launch(c, k_update<ODR>, update_grid(g, c->tile[KID_UPDATE]), c->tile[KID_UPDATE], c->view, c0, c1));
   View out = c->view;
   for (int m = 0; m < 8; m++) out.u[m] = out.uo[m];
-  QL(c, KID_BOUND, k_bound<<<shell_grid(g), BLK, 0, c->stream>>>(out));
+  QL(c, KID_BOUND, launch(c, k_bound<BOUND_STAGE>, shell_grid(g), BLK, out, 0));
   nk += 2;
   return nk;
 }
@@ -768,18 +801,18 @@ long long dsptv_odr(qas_ctx *c, int nc, double nu0, double eta0)
   const double idx = 1.0 / c->grid.dx, idy = 1.0 / c->grid.dy;
   const double idz = g.dim == 3 ? 1.0 / c->grid.dz : 0.0;
   long long nk = 0;
-  QL(c, KID_DBOUND, k_dbound<<<shell_grid(g), BLK, 0, c->stream>>>(c->view, c->d_dctl, nc));
-  QL(c, KID_DCOPY, k_dcopy<<<(unsigned)((g.nd + 255) / 256), 256, 0, c->stream>>>(c->view, c->d_dctl, nc));
+  QL(c, KID_DBOUND, launch(c, k_dbound, shell_grid(g), BLK, c->view, c->d_dctl, nc));
+  QL(c, KID_DCOPY, launch(c, k_dcopy, (unsigned)((g.nd + 255) / 256), 256, c->view, c->d_dctl, nc));
   nk += 2;
   for (int rk = 0; rk < c->scheme.rk; rk++) {
     double c0, c1;
     rk_factors(c->scheme.rk, rk, c0, c1);
-    QL(c, KID_DVEL, k_dvel<<<cells_grid(g), BLK, 0, c->stream>>>(c->view, c->d_dctl, nc));
-    QL(c, KID_ERES, k_eres<ODR><<<cells_grid(g), BLK, 0, c->stream>>>(c->view, c->d_dctl, nc, eta0, idx, idy, idz));
+    QL(c, KID_DVEL, launch(c, k_dvel, cells_grid(g), BLK, c->view, c->d_dctl, nc));
+    QL(c, KID_ERES, launch(c, k_eres<ODR>, cells_grid(g), BLK, c->view, c->d_dctl, nc, eta0, idx, idy, idz));
     QL(c, KID_DFLUX,
-       k_dflux<ODR><<<cells_grid(g), BLK, 0, c->stream>>>(c->view, c->d_dctl, nc, nu0, idx, idy, idz));
-    QL(c, KID_DUPDATE, k_dupdate<ODR><<<update_grid(g), BLK, 0, c->stream>>>(c->view, c->d_dctl, nc, c0, c1));
-    QL(c, KID_DBOUND, k_dbound<<<shell_grid(g), BLK, 0, c->stream>>>(c->view, c->d_dctl, nc));
+       launch(c, k_dflux<ODR>, cells_grid(g), BLK, c->view, c->d_dctl, nc, nu0, idx, idy, idz));
+    QL(c, KID_DUPDATE, launch(c, k_dupdate<ODR>, update_grid(g), BLK, c->view, c->d_dctl, nc, c0, c1));
+    QL(c, KID_DBOUND, launch(c, k_dbound, shell_grid(g), BLK, c->view, c->d_dctl, nc));
     nk += 5;
   }
   return nk;
@@ -806,19 +839,22 @@ long long launch_dissipate(qas_ctx *c, double nu0, double eta0)
   const double dcmax = diss_arrays(c) ? c->diss_dcmax : (dcmax0 > 0.0 ? dcmax0 : 0.0);
   if (!(dcmax > 1e-15)) return 0;
   const double idz = c->grid.dim == 3 ? 1.0 / c->grid.dz : 0.0;
-  QL(c, KID_DSUB, k_dsub_setup<<<1, 1, 0, c->stream>>>(c->view, c->d_dctl, dcmax, c->dr, 1.0 / c->grid.dx,
+  QL(c, KID_DSUB, launch(c, k_dsub_setup, 1, 1, c->view, c->d_dctl, dcmax, c->dr, 1.0 / c->grid.dx,
                                                        1.0 / c->grid.dy, NSUB_CAP, idz));
   long long nk = 1;
   for (int nc = 0; nc < NSUB_CAP; nc++) nk += launch_dsptv(c, nc, nu0, eta0);
   return nk;
 }
 
-long long launch_setdt(qas_ctx *c, double cfl, int rule, double dtrec, int nout)
+// setdt: the reduction (its start value set by k_begin_step, or here with `reset`) and dt in one launch
+long long launch_setdt(qas_ctx *c, double cfl, int rule, double dtrec, int nout, bool reset)
 {
-  QL(c, KID_VMAX, k_vmax_reset<<<1, 1, 0, c->stream>>>(c->view));
-  QL(c, KID_VMAX, k_vmax<<<interior_grid(c->geo), BLK, 0, c->stream>>>(c->view));
-  QL(c, KID_SETDT, k_setdt<<<1, 1, 0, c->stream>>>(c->view, cfl, c->dr, rule, dtrec, nout));
-  return 3;
+  const Geo &g = c->geo;
+  const long long cells = (long long)(g.nx - 2 * GH) * (g.dim >= 2 ? g.ny - 2 * GH : 1) * (g.dim >= 3 ? g.nz - 2 * GH : 1);
+  const unsigned nb = (unsigned)std::min<long long>((cells + 255) / 256, 148 * 8);
+  if (reset) QL(c, KID_VMAX, launch(c, k_vmax_reset<false>, 1, 1, c->view));
+  QL(c, KID_VMAX, launch(c, k_vmax_dt, nb, 256, c->view, cfl, c->dr, rule, dtrec, nout));
+  return reset ? 2 : 1;
 }
 
 // one exec_ iteration
@@ -849,7 +885,7 @@ long long launch_hall(qas_ctx *c, double dt)
       case 3: k_hupdate<3><<<nb, BLK, 0, c->stream>>>(c->view, dtdx, c0, c1); break;
       default: k_hupdate<4><<<nb, BLK, 0, c->stream>>>(c->view, dtdx, c0, c1); break;
     }
-    k_bound<<<shell_grid(g), BLK, 0, c->stream>>>(c->view);
+    launch(c, k_bound<BOUND_STAGE>, shell_grid(g), BLK, c->view, 0);
     nk += 5;
   }
   return nk;
@@ -874,7 +910,7 @@ long long launch_hall_subcycles(qas_ctx *c, double cfl)
   long long nk = 1;
   for (int h = 0; h < hmax; h++) {
     nk += launch_hall(c, dt / hmax);
-    k_bound<<<shell_grid(c->geo), BLK, 0, c->stream>>>(c->view);
+    launch(c, k_bound<BOUND_STAGE>, shell_grid(c->geo), BLK, c->view, 0);
     nk++;
   }
   return nk;
@@ -882,15 +918,20 @@ long long launch_hall_subcycles(qas_ctx *c, double cfl)
 
 bool hall_active(const qas_ctx *c) { return c->hall && c->hall_di != 0; }
 
-long long launch_exec_step(qas_ctx *c, const qas_run_opts &o, int n_after)
+// the state's ghosts are as the last stage of the previous step filled them, unless a driver changes
+// the state in between (gravity's setdt rounds the energy, Hall sub-cycles start from a fill)
+bool ghosts_kept(const qas_ctx *c) { return !c->view.phi && !hall_active(c); }
+
+// fill: the ghost fill at the start of the step
+long long launch_exec_step(qas_ctx *c, const qas_run_opts &o, int n_after, bool fill = true)
 {
   long long nk = 0;
-  QL(c, KID_BEGIN, k_begin_step<<<1, 1, 0, c->stream>>>(c->view, o.stop_rule == 2 ? 0 : 1));
-  QL(c, KID_BOUND, k_bound<<<shell_grid(c->geo), BLK, 0, c->stream>>>(c->view));
+  QL(c, KID_BEGIN, launch(c, k_begin_step, 1, 1, c->view, o.stop_rule == 2 ? 0 : 1));
+  if (fill) QL(c, KID_BOUND, launch(c, k_bound<BOUND_STAGE>, shell_grid(c->geo), BLK, c->view, 0));
   if (hall_active(c)) nk += launch_hall_subcycles(c, o.cfl);
-  nk += 2 + launch_ideal(c);
+  nk += 1 + (fill ? 1 : 0) + launch_ideal(c);
   if (c->grid.dim >= 2 && (o.nu0 > 0.0 || o.eta0 > 0.0 || diss_arrays(c))) nk += launch_dissipate(c, o.nu0, o.eta0);
-  if (o.flg && (n_after % 2 == 0)) nk += launch_setdt(c, o.cfl, o.stop_rule, o.dtrec, o.nout);
+  if (o.flg && (n_after % 2 == 0)) nk += launch_setdt(c, o.cfl, o.stop_rule, o.dtrec, o.nout, false);
   return nk;
 }
 
@@ -911,6 +952,12 @@ qas_status read_ctl(qas_ctx *c)
   return QAS_OK;
 }
 
+// queued: h_ctl must stay as it is until the stream's next synchronisation
+qas_status queue_ctl(qas_ctx *c)
+{
+  QAS_CUDA(cudaMemcpyAsync(c->d_ctl, c->h_ctl, sizeof(Ctl), cudaMemcpyHostToDevice, c->stream));
+  return QAS_OK;
+}
 qas_status write_ctl(qas_ctx *c)
 {
   QAS_CUDA(cudaMemcpyAsync(c->d_ctl, c->h_ctl, sizeof(Ctl), cudaMemcpyHostToDevice, c->stream));
@@ -1224,8 +1271,7 @@ qas_status qas_bound(qas_ctx *c)
 {
   QAS_API_TRY
   if (!c) return QAS_ERR_INVALID;
-  QAS_CUDA(cudaMemsetAsync(&c->d_ctl->done, 0, sizeof(int), c->stream));
-  k_bound<<<shell_grid(c->geo), BLK, 0, c->stream>>>(c->view);
+  launch(c, k_bound<BOUND_CALL>, shell_grid(c->geo), BLK, c->view, 0);
   c->launches++;
   return check_launch(c);
   QAS_API_CATCH
@@ -1235,9 +1281,8 @@ qas_status qas_step(qas_ctx *c, double dt)
 {
   QAS_API_TRY
   if (!c) return QAS_ERR_INVALID;
-  // a single ideal(dt): make sure the loop's done flag does not mask the kernels
-  QAS_CUDA(cudaMemsetAsync(&c->d_ctl->done, 0, sizeof(int), c->stream));
-  k_set_dt<<<1, 1, 0, c->stream>>>(c->view, dt);
+  // a single ideal(dt): k_set_dt takes back the loop's stop flag, which would mask the kernels
+  launch(c, k_set_dt, 1, 1, c->view, dt);
   c->launches += 1 + launch_ideal(c);
   return check_launch(c);
   QAS_API_CATCH
@@ -1247,9 +1292,8 @@ qas_status qas_cfl_vmax(qas_ctx *c, double *vmax)
 {
   QAS_API_TRY
   if (!c || !vmax) return QAS_ERR_INVALID;
-  QAS_CUDA(cudaMemsetAsync(&c->d_ctl->done, 0, sizeof(int), c->stream));
-  k_vmax_reset<<<1, 1, 0, c->stream>>>(c->view);
-  k_vmax<<<interior_grid(c->geo), BLK, 0, c->stream>>>(c->view);
+  launch(c, k_vmax_reset<true>, 1, 1, c->view);
+  launch(c, k_vmax, interior_grid(c->geo), BLK, c->view);
   c->launches += 2;
   qas_status s = check_launch(c);
   if (s != QAS_OK) return s;
@@ -1298,24 +1342,28 @@ qas_status qas_run(qas_ctx *c, const qas_run_opts *opts, qas_run_info *info)
     c->h_ctl->first = 1;
     c->h_ctl->nmax = INT_MAX;
     c->h_ctl->tmax = o.stop_rule == 0 ? INFINITY : o.dtrec * o.nout;
-    if ((s = write_ctl(c)) != QAS_OK) return s;
-    c->launches += launch_setdt(c, o.cfl, o.stop_rule, o.dtrec, o.nout);
+    if ((s = queue_ctl(c)) != QAS_OK) return s;
+    c->launches += launch_setdt(c, o.cfl, o.stop_rule, o.dtrec, o.nout, true);
     if ((s = check_launch(c)) != QAS_OK) return s;
     c->run_initialised = true;
   } else {
     if ((s = read_ctl(c)) != QAS_OK) return s;
     c->h_ctl->done = 0;
     if (o.stop_rule == 0) c->h_ctl->nmax = INT_MAX;
-    if ((s = write_ctl(c)) != QAS_OK) return s;
+    if ((s = queue_ctl(c)) != QAS_OK) return s;
   }
-  if ((s = read_ctl(c)) != QAS_OK) return s;
   const int n0 = c->h_ctl->n;
   int n_host = n0;
   const int limit = o.max_steps > 0 ? o.max_steps : INT_MAX;
   int launched = 0;
+  const bool fill = !ghosts_kept(c);
+  if (!fill) {  // once for all steps of the call
+    launch(c, k_bound<BOUND_START>, shell_grid(c->geo), BLK, c->view, o.stop_rule == 2 ? 0 : 1);
+    c->launches++;
+  }
   // odd n: one eager step so graphs always start at an even n
   if (n_host % 2 == 1 && launched < limit) {
-    c->launches += launch_exec_step(c, o, n_host + 1);
+    c->launches += launch_exec_step(c, o, n_host + 1, fill);
     n_host++;
     launched++;
   }
@@ -1331,7 +1379,9 @@ qas_status qas_run(qas_ctx *c, const qas_run_opts *opts, qas_run_info *info)
       }
       cudaGraph_t gph;
       QAS_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-      long long nk = launch_exec_step(c, o, 1) + launch_exec_step(c, o, 2);
+      c->capturing = true;
+      long long nk = launch_exec_step(c, o, 1, fill) + launch_exec_step(c, o, 2, fill);
+      c->capturing = false;
       cudaError_t e = cudaStreamEndCapture(c->stream, &gph);
       if (e != cudaSuccess) return cuda_fail(e, "graph capture");
       e = cudaGraphInstantiate(&c->graph, gph, 0);
@@ -1358,7 +1408,7 @@ qas_status qas_run(qas_ctx *c, const qas_run_opts *opts, qas_run_info *info)
         n_host += 2;
         this_chunk += 2;
       } else {
-        c->launches += launch_exec_step(c, o, n_host + 1);
+        c->launches += launch_exec_step(c, o, n_host + 1, fill);
         launched++;
         n_host++;
         this_chunk++;
@@ -1392,10 +1442,10 @@ qas_status qas_dsptv(qas_ctx *c, double dt, double nu0, double eta0)
   const Geo &g = c->geo;
   const double idx = 1.0 / c->grid.dx, idy = 1.0 / c->grid.dy;
   const double idz = g.dim == 3 ? 1.0 / c->grid.dz : 0.0;
-  k_dsub_fixed<<<1, 1, 0, c->stream>>>(c->view, c->d_dctl, dt, idx, idy, idz);
+  launch(c, k_dsub_fixed, 1, 1, c->view, c->d_dctl, dt, idx, idy, idz);
   // dsptv itself does not fill the ghosts first; launch_dsptv starts with a fill, so
   // run the body without it: copy, stages
-  k_dcopy<<<(unsigned)((g.nd + 255) / 256), 256, 0, c->stream>>>(c->view, c->d_dctl, 0);
+  launch(c, k_dcopy, (unsigned)((g.nd + 255) / 256), 256, c->view, c->d_dctl, 0);
   long long nk = 2;
   for (int rk = 0; rk < c->scheme.rk; rk++) {
     double c0, c1;
@@ -1403,11 +1453,11 @@ qas_status qas_dsptv(qas_ctx *c, double dt, double nu0, double eta0)
     switch (c->scheme.odr) {
 #define QAS_DST(O)                                                                                        \
   case O:                                                                                                 \
-    k_dvel<<<cells_grid(g), BLK, 0, c->stream>>>(c->view, c->d_dctl, 0);                                  \
-    k_eres<O><<<cells_grid(g), BLK, 0, c->stream>>>(c->view, c->d_dctl, 0, eta0, idx, idy, idz);          \
-    k_dflux<O><<<cells_grid(g), BLK, 0, c->stream>>>(c->view, c->d_dctl, 0, nu0, idx, idy, idz);          \
-    k_dupdate<O><<<update_grid(g), BLK, 0, c->stream>>>(c->view, c->d_dctl, 0, c0, c1);                   \
-    k_dbound<<<shell_grid(g), BLK, 0, c->stream>>>(c->view, c->d_dctl, 0);                                \
+    launch(c, k_dvel, cells_grid(g), BLK, c->view, c->d_dctl, 0);                                  \
+    launch(c, k_eres<O>, cells_grid(g), BLK, c->view, c->d_dctl, 0, eta0, idx, idy, idz);          \
+    launch(c, k_dflux<O>, cells_grid(g), BLK, c->view, c->d_dctl, 0, nu0, idx, idy, idz);          \
+    launch(c, k_dupdate<O>, update_grid(g), BLK, c->view, c->d_dctl, 0, c0, c1);                   \
+    launch(c, k_dbound, shell_grid(g), BLK, c->view, c->d_dctl, 0);                                \
     break;
       QAS_DST(1)
       QAS_DST(2)
@@ -1429,8 +1479,7 @@ qas_status qas_dissipate(qas_ctx *c, double dt, double nu0, double eta0)
   if (!c) return QAS_ERR_INVALID;
   if (c->grid.dim < 2 || c->view.phi) return QAS_ERR_UNSUPPORTED;
   if (diss_arrays(c) && (nu0 != 0.0 || eta0 != 0.0)) return QAS_ERR_INVALID;
-  QAS_CUDA(cudaMemsetAsync(&c->d_ctl->done, 0, sizeof(int), c->stream));
-  k_set_dt<<<1, 1, 0, c->stream>>>(c->view, dt);
+  launch(c, k_set_dt, 1, 1, c->view, dt);
   c->launches += 1 + launch_dissipate(c, nu0, eta0);
   return check_launch(c);
   QAS_API_CATCH

@@ -21,6 +21,7 @@ struct DCtl {
 __global__ void k_dsub_setup(View v, DCtl *dc, double dcmax, double dr, double idx, double idy, int cap,
                              double idz = 0.0)
 {
+  pdl_begin();
   if (v.ctl->done) return;
   const double dt = v.ctl->dt;
   int ncmax = 0;
@@ -39,6 +40,7 @@ __global__ void k_dsub_setup(View v, DCtl *dc, double dcmax, double dr, double i
 // host-supplied dt for one dsptv(dt) call
 __global__ void k_dsub_fixed(View v, DCtl *dc, double dt, double idx, double idy, double idz)
 {
+  pdl_begin();
   dc->ncmax = 1;
   dc->sdt = dt;
   dc->sdtd[0] = dt * idx;
@@ -46,7 +48,8 @@ __global__ void k_dsub_fixed(View v, DCtl *dc, double dt, double idx, double idy
   dc->sdtd[2] = dt * idz;
 }
 
-#define QAS_DSUB_GUARD()                        \
+#define QAS_DSUB_GUARD() \
+  pdl_begin();           \
   if (v.ctl->done || nc >= dc->ncmax) return;
 
 // velocity at every cell (vlcty, common/mhd_class.hpp:59-65)

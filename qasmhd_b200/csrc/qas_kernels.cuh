@@ -68,7 +68,7 @@ struct Ctl {
   unsigned long long vmax_bits;  // setdt reduction (positive doubles order like their bits)
   int n, nmax, done, first;
   int err;                       // latched device error bits
-  int pad;
+  unsigned ticket;               // blocks of k_vmax_dt that are done (0 between launches)
 };
 
 // Ghost-fill maps: for group G (0 state, 1 cell-centre B, 2 dv), field m, axis a and
@@ -108,6 +108,16 @@ struct View {
   int recon;  // face-value reconstruction: 0 characteristic (mhd_m/a_reconst), 1 primitive (mhd_reconst),
               // 2 Athena-type characteristic (mhd_c_reconst)
 };
+
+// First statement of every kernel launched with programmatic stream serialization: the next kernel
+// of the stream may take its place on the SMs as soon as every block of this one has started (the
+// last wave's free slots, all of it on a small grid), and nothing is read or written before every
+// earlier kernel of the stream has finished.
+__device__ __forceinline__ void pdl_begin()
+{
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+}
 
 __device__ __forceinline__ long long cidx(const Geo &g, int i, int j, int k)
 {
@@ -244,6 +254,7 @@ __device__ __forceinline__ void prim_body(const View &v, int i, int j, int k)
 template <int ODR>
 __global__ void QAS_PRIM_BOUNDS k_prim(View v)
 {
+  pdl_begin();
   if (v.ctl->done) return;
   QAS_CELL_INDEX();
   prim_body<ODR>(v, i, j, k);
@@ -289,6 +300,7 @@ __device__ __forceinline__ void dv_body(const View &v, int i, int j, int k)
 }
 __global__ void k_dv(View v)
 {
+  pdl_begin();
   if (v.ctl->done) return;
   QAS_CELL_INDEX();
   dv_body(v, i, j, k);
@@ -430,6 +442,7 @@ __device__ __forceinline__ void lr_body(const View &v, int i, int j, int k)
 template <int ODR, int A, int PR = 0>
 __global__ void __launch_bounds__(128, QAS_LR_MINB) k_lr(const __grid_constant__ View v)
 {
+  pdl_begin();
   if (v.ctl->done) return;
   QAS_CELL_INDEX();
   lr_body<ODR, A, PR>(v, i, j, k);
@@ -549,6 +562,7 @@ __device__ __forceinline__ void flux_body(const View &v, int i, int j, int k)
 template <int RMN, int A>
 __global__ void __launch_bounds__(128, QAS_FLUX_MINB_OF(RMN)) k_flux(View v)
 {
+  pdl_begin();
   if (v.ctl->done) return;
   QAS_CELL_INDEX();
   flux_body<RMN, A>(v, i, j, k);
@@ -562,6 +576,7 @@ __global__ void __launch_bounds__(128, QAS_FLUX_MINB_OF(RMN)) k_flux(View v)
 template <int A>
 __global__ void __launch_bounds__(128, QAS_FLUX_MLAU_MINB) k_flux_mlau(View v)
 {
+  pdl_begin();
   if (v.ctl->done) return;
   QAS_CELL_INDEX();
   flux_body<3, A>(v, i, j, k);
@@ -706,6 +721,7 @@ __device__ __forceinline__ void sweep_x_cell(const View &v, int i, int j, int k,
 template <int ODR, int RMN, int PR>
 __global__ void __launch_bounds__(SWB, QAS_SWEEP_MINB_OF(RMN)) k_sweep_x(const __grid_constant__ View v, long long nwarps)
 {
+  pdl_begin();
   if (v.ctl->done) return;
   __shared__ double sm[SLOTS * SLP];
   const Geo &g = v.g;
@@ -769,6 +785,7 @@ __device__ __forceinline__ void sweep_columns(const View &v, int i, int o, bool 
 template <int ODR, int RMN, int A, int PR>
 __global__ void __launch_bounds__(SWB, QAS_SWEEP_MINB_OF(RMN)) k_sweep_m(const __grid_constant__ View v, int seg)
 {
+  pdl_begin();
   if (v.ctl->done) return;
   const Geo &g = v.g;
   __shared__ double sm[SLOTS * SLP];
@@ -857,6 +874,7 @@ __device__ __forceinline__ void emf_body(const View &v, int i, int j, int k)
 template <int ODR>
 __global__ void QAS_EMF_BOUNDS k_emf(View v)
 {
+  pdl_begin();
   if (v.ctl->done) return;
   QAS_CELL_INDEX();
   emf_body<ODR>(v, i, j, k);
@@ -977,6 +995,7 @@ __device__ __forceinline__ bool update_cell(const Geo &g, int ti, int tj, int tk
 template <int ODR>
 __global__ void QAS_UPDATE_BOUNDS k_update(View v, double c0, double c1)
 {
+  pdl_begin();
   if (v.ctl->done) return;
   int i, j, k;
   if (!update_cell(v.g, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y,
@@ -1071,10 +1090,26 @@ __device__ __forceinline__ void bound_body(const View &v, int i, int j, int k)
     if (wr[m]) v.u[m][c] = nv[m];
 }
 
-__global__ void k_bound(View v)
+// the while() test of exec_
+__device__ __forceinline__ bool run_goes_on(const Ctl *c, int check_tim)
 {
-  if (v.ctl->done) return;
+  return check_tim ? (c->n < c->nmax && c->tim < c->tmax) : (c->n < c->nmax);
+}
+
+// MODE 0: within a step; 1: before the first step of a run call, which may turn out to have none left
+// (the later steps find the ghosts as the last stage filled them); 2: a call of its own, which also
+// takes back the stop flag
+enum { BOUND_STAGE, BOUND_START, BOUND_CALL };
+template <int MODE>
+__global__ void k_bound(View v, int check_tim)
+{
+  pdl_begin();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (MODE == BOUND_CALL) {
+    if (t == 0) v.ctl->done = 0;
+  } else if (v.ctl->done || (MODE == BOUND_START && !run_goes_on(v.ctl, check_tim))) {
+    return;
+  }
   if (t >= shell_cells(v.g)) return;
   int i, j, k;
   shell_cell(v.g, t, i, j, k);
@@ -1089,8 +1124,7 @@ __device__ __forceinline__ void begin_body(const View &v, int check_tim)
 {
   Ctl *c = v.ctl;
   if (c->done) return;
-  const bool go = check_tim ? (c->n < c->nmax && c->tim < c->tmax) : (c->n < c->nmax);
-  if (!go) {
+  if (!run_goes_on(c, check_tim)) {
     c->done = 1;
     return;
   }
@@ -1099,22 +1133,35 @@ __device__ __forceinline__ void begin_body(const View &v, int check_tim)
   c->dtd[0] = c->dt / v.dx;
   c->dtd[1] = v.g.dim >= 2 ? c->dt / v.dy : 0.0;
   c->dtd[2] = v.g.dim >= 3 ? c->dt / v.dz : 0.0;
+  c->vmax_bits = (unsigned long long)__double_as_longlong(1.0);  // for the setdt after this step
 }
-__global__ void k_begin_step(View v, int check_tim) { begin_body(v, check_tim); }
+__global__ void k_begin_step(View v, int check_tim)
+{
+  pdl_begin();
+  begin_body(v, check_tim);
+}
 
-// dt/dx etc. for a host-supplied dt (qas_step)
+// dt/dx etc. for a host-supplied dt (a call of its own: qas_step), the stop flag taken back
 __global__ void k_set_dt(View v, double dt)
 {
+  pdl_begin();
   Ctl *c = v.ctl;
+  c->done = 0;
   c->dt = dt;
   c->dtd[0] = dt / v.dx;
   c->dtd[1] = v.g.dim >= 2 ? dt / v.dy : 0.0;
   c->dtd[2] = v.g.dim >= 3 ? dt / v.dz : 0.0;
 }
 
+// CALL: a call of its own, which takes the stop flag back
+template <bool CALL>
 __global__ void k_vmax_reset(View v)
 {
-  if (v.ctl->done) return;
+  pdl_begin();
+  if (CALL)
+    v.ctl->done = 0;
+  else if (v.ctl->done)
+    return;
   v.ctl->vmax_bits = (unsigned long long)__double_as_longlong(1.0);
 }
 
@@ -1159,6 +1206,7 @@ __device__ __forceinline__ double vmax_cell(const View &v, int i, int j, int k)
 // (mhd2d_class.cpp:17-26); NaN never wins, as with `if (vtmp > vmax)`.
 __global__ void k_vmax(View v)
 {
+  pdl_begin();
   if (v.ctl->done) return;
   const Geo &g = v.g;
   const int i = GH + blockIdx.x * blockDim.x + threadIdx.x;
@@ -1195,7 +1243,7 @@ __device__ __forceinline__ void setdt_body(const View &v, double cfl, double dr,
 {
   Ctl *c = v.ctl;
   if (c->done) return;
-  const double vmax = __longlong_as_double((long long)c->vmax_bits);
+  const double vmax = __longlong_as_double((long long)__ldcg(&c->vmax_bits));  // from L2, where the atomics are
   c->dt = cfl * dr / vmax;
   if (c->first) {
     if (rule == 2) {
@@ -1209,7 +1257,43 @@ __device__ __forceinline__ void setdt_body(const View &v, double cfl, double dr,
 }
 __global__ void k_setdt(View v, double cfl, double dr, int rule, double dtrec, int nout)
 {
+  pdl_begin();
   setdt_body(v, cfl, dr, rule, dtrec, nout);
+}
+
+// k_vmax and k_setdt in one launch: blocks stride over the interior, the last one to finish sets dt
+__global__ void k_vmax_dt(View v, double cfl, double dr, int rule, double dtrec, int nout)
+{
+  pdl_begin();
+  if (v.ctl->done) return;
+  const Geo &g = v.g;
+  const long long mx = g.nx - 2 * GH, my = g.dim >= 2 ? g.ny - 2 * GH : 1, mz = g.dim >= 3 ? g.nz - 2 * GH : 1;
+  double best = 1.0;
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < mx * my * mz;
+       t += (long long)gridDim.x * blockDim.x) {
+    const long long r = t / mx;
+    const double vt = vmax_cell(v, GH + (int)(t - r * mx), (g.dim >= 2 ? GH : 0) + (int)(r % my),
+                                (g.dim >= 3 ? GH : 0) + (int)(r / my));
+    if (vt > best) best = vt;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double other = __shfl_xor_sync(0xffffffffu, best, o);
+    best = (other > best) ? other : best;
+  }
+  __shared__ double red[32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (lane == 0) red[wid] = best;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < (int)(blockDim.x >> 5); w++) best = (red[w] > best) ? red[w] : best;
+  atomicMax(&v.ctl->vmax_bits, (unsigned long long)__double_as_longlong(best));
+  __threadfence();
+  if (atomicAdd(&v.ctl->ticket, 1u) == gridDim.x - 1) {
+    v.ctl->ticket = 0;
+    __threadfence();
+    setdt_body(v, cfl, dr, rule, dtrec, nout);
+  }
 }
 
 // |div B| with df1[ODR-1] over the interior; max by bit pattern of non-negative doubles

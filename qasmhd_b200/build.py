@@ -13,11 +13,12 @@ import os
 import shutil
 import subprocess
 import sys
+import tempfile
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libqas.so")
-SOURCES = ["qas_api.cu"]
+SOURCES = ["qas_api.cu", "qas_sweep.cu"]
 HEADERS = ["qas_device.cuh", "qas_kernels.cuh", "qas_dissip.cuh", "qas_batch.cuh", "qas_batch_api.inc",
            "qas_adjoint.cuh", "qas_adjoint_kernels.cuh", "qas_adjoint_api.inc", "qas_noalloc.inc",
            "qas_io.inc", "qas_tma.cuh", "qas_dd.inc", "qas_hall.cuh", "qas_pipe.cuh", "qas_pipe.inc"]
@@ -25,7 +26,7 @@ HEADERS = ["qas_device.cuh", "qas_kernels.cuh", "qas_dissip.cuh", "qas_batch.cuh
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "--fmad=false", "-lineinfo", "-std=c++17",
-    "-Xcompiler", "-fPIC", "-shared", "-cudart=static",
+    "-Xcompiler", "-fPIC", "-cudart=static",
 ]
 
 
@@ -48,10 +49,19 @@ def _stale() -> bool:
 def build_library(force: bool = False, verbose: bool = False) -> str:
     if not force and not _stale():
         return LIB
-    cmd = [nvcc(), *NVCC_FLAGS, "-o", LIB] + [os.path.join(CSRC, s) for s in SOURCES]
-    if verbose:
-        print(" ".join(cmd), flush=True)
-    subprocess.run(cmd, check=True, cwd=CSRC)
+    with tempfile.TemporaryDirectory(prefix="qasbuild_") as tmp:  # the units side by side, then one library
+        objs = [os.path.join(tmp, os.path.splitext(s)[0] + ".o") for s in SOURCES]
+        cmds = [[nvcc(), *NVCC_FLAGS, "-DQAS_SEPARATE_UNITS", "-c", "-o", o, os.path.join(CSRC, s)]
+                for s, o in zip(SOURCES, objs)]
+        link = [nvcc(), *NVCC_FLAGS, "-shared", "-o", LIB, *objs]
+        if verbose:
+            print("\n".join(" ".join(c) for c in cmds + [link]), flush=True)
+        procs = [subprocess.Popen(c, cwd=CSRC) for c in cmds]
+        codes = [p.wait() for p in procs]
+        for c, rc in zip(cmds, codes):
+            if rc != 0:
+                raise subprocess.CalledProcessError(rc, c)
+        subprocess.run(link, check=True, cwd=CSRC)
     return LIB
 
 

@@ -24,6 +24,9 @@
 #include "qas_tma.cuh"
 #include "qas_hall.cuh"
 #include "qas_pipe.cuh"
+#ifndef QAS_SEPARATE_UNITS  // the build compiles these side by side
+#include "qas_sweep.cu"
+#endif
 
 using namespace qas;
 
@@ -328,15 +331,17 @@ long long pdl_launch(cudaError_t &err, void (*kern)(KArgs...), dim3 grid, dim3 b
   return 1;
 }
 
-// one kernel on the context's stream; issued eagerly with programmatic stream serialization, which hides
-// the launch latency behind the kernel before (OT 128x96: 389 -> 267 us for two steps of single calls),
-// in a graph with plain edges, which are the faster ones there (OT 200^2: 150 against 165 us a step).
-// Only kernels that begin with pdl_begin().  An error stays with the runtime (check_launch)
+// one kernel on the context's stream with programmatic stream serialization, which hides the launch behind
+// the kernel before; a graph of a small grid keeps plain edges, between its short kernels the faster ones.
+// Two steps of single calls on OT 128x96 389 -> 267 us; in a graph, us a step, plain / programmatic edges: OT
+// 200^2 150 / 165, RT 128x512 (71 k cells) 190 / 198, KH 515x301 (161 k) 646 / 634, KH 512^2 400 / 383, OT
+// 1024^2 1211 / 1198.  Only kernels that begin with pdl_begin().  An error stays with the runtime
+// (check_launch)
 template <class... KArgs, class... Args>
 void launch(qas_ctx *c, void (*kern)(KArgs...), dim3 grid, dim3 block, Args... args)
 {
   cudaError_t e = cudaSuccess;
-  if (c->capturing)
+  if (c->capturing && c->geo.nd < (1 << 17))
     kern<<<grid, block, 0, c->stream>>>(args...);
   else
     pdl_launch(e, kern, grid, block, c->stream, args...);
@@ -572,66 +577,67 @@ int sweep_seg(qas_ctx *c, int a, const void *fn)
   return bseg;
 }
 
-// choose the y / z segment lengths outside any stream capture (occupancy query); the fused
-// sweeps are built for 4th-order interpolation only (other orders take the two-kernel form)
-template <int RMN>
-void sweep_prepare_t(qas_ctx *c)
+// the fused sweeps are built for the 2nd and the 4th order (the others take the two-kernel form), the
+// Athena-type reconstruction for the 4th
+bool sweep_built(const qas_ctx *c) { return c->scheme.odr == 4 || (c->scheme.odr == 2 && c->scheme.char_mode != 2); }
+SweepFn sweep_fn(const qas_ctx *c, int a)
 {
-  if (c->geo.dim >= 2) sweep_seg(c, 1, (const void *)k_sweep_m<4, RMN, 1, 0>);
-  if (c->geo.dim >= 3) sweep_seg(c, 2, (const void *)k_sweep_m<4, RMN, 2, 0>);
+  return sweep_kernel(c->scheme.odr, c->scheme.rmn, c->scheme.char_mode == 2, c->scheme.odr == 2 ? 7 : 1 << a);
 }
+// choose the y / z segment lengths outside any stream capture (occupancy query)
 void sweep_prepare(qas_ctx *c)
 {
-  if (c->scheme.odr != 4) return;
-  switch (c->scheme.rmn) {
-    case 0: sweep_prepare_t<0>(c); break;
-    case 1: sweep_prepare_t<1>(c); break;
-    case 2: sweep_prepare_t<2>(c); break;
-    default: sweep_prepare_t<3>(c); break;
-  }
+  if (!sweep_built(c)) return;
+  if (c->geo.dim >= 2) sweep_seg(c, 1, (const void *)sweep_fn(c, 1));
+  if (c->geo.dim >= 3) sweep_seg(c, 2, (const void *)sweep_fn(c, 2));
 }
 
 // the axes whose face states stay on chip by default (bit a).  3D: all.  2D: x, and y for the HLLD
 // solvers and on small grids, where a launch counts more than the march (OT / KH 1024^2, two kernels
 // against one, us: x HLLD 139 / 121, LHLLD 149 / 134, MLAU 152 / 139, Roe 162 / 162; y HLLD 138 / 136,
-// LHLLD 152 / 147, MLAU 147 / 157, Roe 161 / 178).  1D and the other orders: none.
+// LHLLD 152 / 147, MLAU 147 / 157, Roe 161 / 178).  1D: none.
 unsigned fused_axes(const qas_ctx *c)
 {
-  if (c->scheme.odr != 4 || c->geo.dim == 1) return 0u;
-  if (c->geo.dim == 3) return 7u;
+  if (!sweep_built(c) || c->geo.dim == 1) return 0u;
+  if (c->geo.dim == 3 || c->scheme.odr == 2) return 7u;
   const bool hlld = c->scheme.rmn == 1 || c->scheme.rmn == 2;
   return hlld || c->geo.nd <= (1ll << 18) ? 3u : 1u;
 }
 
-template <int RMN, int PR>
-void launch_sweep_pr(qas_ctx *c, int a)
+// the blocks of a sweep over the axes
+unsigned sweep_plan(qas_ctx *c, unsigned axes, SweepPlan &pl)
 {
   const Geo &g = c->geo;
-  if (a == 0) {
+  pl = SweepPlan{};
+  for (int a = 1; a < g.dim; a++) {
+    if (!((axes >> a) & 1)) continue;
+    const int seg = sweep_seg(c, a, (const void *)sweep_fn(c, a)), len = g.n[a] - 5;
+    pl.cols[a - 1] = (unsigned)(((long long)g.nx * (a == 1 ? g.nz : g.ny) + 31) / 32);
+    pl.seg[a - 1] = seg;
+    pl.bq[a - 1] = pl.cols[a - 1] * (unsigned)((len + seg - 1) / seg);
+  }
+  unsigned nbx = 0;
+  if (axes & 1) {
     // warp w takes flattened cells [31w, 31w+32); the last cell needing a flux is total-1
     const long long total = (long long)(g.nx - 4) * g.ny * g.nz;
-    const long long nwarps = (total - 2) / 31 + 1;
-    const unsigned nb = (unsigned)((nwarps + SWB / 32 - 1) / (SWB / 32));
-    QL(c, KID_SWEEP, launch(c, k_sweep_x<4, RMN, PR>, nb, SWB, c->view, nwarps));
-    return;
+    pl.nwarps = (total - 2) / 31 + 1;
+    nbx = (unsigned)((pl.nwarps + SWB / 32 - 1) / (SWB / 32));
   }
-  const unsigned colb = (unsigned)(((long long)g.nx * (a == 1 ? g.nz : g.ny) + 31) / 32);
-  const int len = g.n[a] - 5;
-  if (a == 1) {
-    const int seg = sweep_seg(c, 1, (const void *)k_sweep_m<4, RMN, 1, 0>);
-    QL(c, KID_SWEEP, launch(c, k_sweep_m<4, RMN, 1, PR>, dim3(colb, (len + seg - 1) / seg), SWB, c->view, seg));
-  } else {
-    const int seg = sweep_seg(c, 2, (const void *)k_sweep_m<4, RMN, 2, 0>);
-    QL(c, KID_SWEEP, launch(c, k_sweep_m<4, RMN, 2, PR>, dim3(colb, (len + seg - 1) / seg), SWB, c->view, seg));
-  }
+  return nbx + pl.bq[0] + pl.bq[1];
 }
-template <int RMN>
-void launch_sweep(qas_ctx *c, int a)
+// the fused axes of a stage: together at the 2nd order, else one after the other; returns the launches
+long long launch_sweep(qas_ctx *c, unsigned axes)
 {
-  if (c->view.recon != 2)
-    launch_sweep_pr<RMN, 0>(c, a);
-  else
-    launch_sweep_pr<RMN, -1>(c, a);
+  long long nk = 0;
+  for (int a = 0; a < c->geo.dim; a++) {
+    const unsigned ax = c->scheme.odr == 2 ? axes : axes & (1u << a);
+    if (!ax || (nk && c->scheme.odr == 2)) continue;
+    SweepPlan pl;
+    const unsigned nb = sweep_plan(c, ax, pl);
+    QL(c, KID_SWEEP, launch(c, sweep_fn(c, a), nb, SWB, c->view, pl));
+    nk++;
+  }
+  return nk;
 }
 
 // HMHD1D::crcte on the by and bz fluxes (1D Hall driver with electron inertia), after the
@@ -684,20 +690,12 @@ long long stage_rest(qas_ctx *c, double c0, double c1)
 {
   const Geo &g = c->geo;
   long long nk = 0;
+  // a profile run keeps the 2D stage's two kernels apart, to time each
+  const bool split = !sweep_built(c) || (c->prof && g.dim == 2 && !c->fused_set);
+  const unsigned axes = split ? 0u : c->fused & ((1u << g.dim) - 1u);
+  if (axes) nk += launch_sweep(c, axes);
   for (int a = 0; a < g.dim; a++) {
-    if constexpr (ODR == 4) {
-      // a profile run keeps the 2D stage's two kernels apart, to time each
-      if (((c->fused >> a) & 1) && !(c->prof && g.dim == 2 && !c->fused_set)) {
-        switch (c->scheme.rmn) {
-          case 0: launch_sweep<0>(c, a); break;
-          case 1: launch_sweep<1>(c, a); break;
-          case 2: launch_sweep<2>(c, a); break;
-          default: launch_sweep<3>(c, a); break;
-        }
-        nk += 1;
-        continue;
-      }
-    }
+    if ((axes >> a) & 1) continue;
     launch_lr<ODR>(c, a);
     switch (c->scheme.rmn) {
       case 0: launch_flux<0>(c, a); break;
@@ -1326,6 +1324,20 @@ qas_status qas_run_reset(qas_ctx *c)
   QAS_API_CATCH
 }
 
+static qas_status end_run(qas_ctx *c, int n0, qas_run_info *info)
+{
+  const qas_status s = read_ctl(c);
+  if (s != QAS_OK) return s;
+  if (info) {
+    info->steps = c->h_ctl->n - n0;
+    info->n = c->h_ctl->n;
+    info->nmax = c->h_ctl->nmax;
+    info->tim = c->h_ctl->tim;
+    info->dt = c->h_ctl->dt;
+  }
+  return QAS_OK;
+}
+
 qas_status qas_run(qas_ctx *c, const qas_run_opts *opts, qas_run_info *info)
 {
   QAS_API_TRY
@@ -1420,15 +1432,7 @@ qas_status qas_run(qas_ctx *c, const qas_run_opts *opts, qas_run_info *info)
       if (c->h_ctl->done) break;
     }
   }
-  if ((s = read_ctl(c)) != QAS_OK) return s;
-  if (info) {
-    info->steps = c->h_ctl->n - n0;
-    info->n = c->h_ctl->n;
-    info->nmax = c->h_ctl->nmax;
-    info->tim = c->h_ctl->tim;
-    info->dt = c->h_ctl->dt;
-  }
-  return QAS_OK;
+  return end_run(c, n0, info);
   QAS_API_CATCH
 }
 

@@ -18,7 +18,7 @@ struct DCtl {
 };
 
 // setdc + ncmax = 1 + (int)(2*(dcmax*dt)/(dr*dr))
-__global__ void k_dsub_setup(View v, DCtl *dc, double dcmax, double dr, double idx, double idy, int cap,
+static __global__ void k_dsub_setup(View v, DCtl *dc, double dcmax, double dr, double idx, double idy, int cap,
                              double idz = 0.0)
 {
   pdl_begin();
@@ -38,7 +38,7 @@ __global__ void k_dsub_setup(View v, DCtl *dc, double dcmax, double dr, double i
 }
 
 // host-supplied dt for one dsptv(dt) call
-__global__ void k_dsub_fixed(View v, DCtl *dc, double dt, double idx, double idy, double idz)
+static __global__ void k_dsub_fixed(View v, DCtl *dc, double dt, double idx, double idy, double idz)
 {
   pdl_begin();
   dc->ncmax = 1;
@@ -53,24 +53,27 @@ __global__ void k_dsub_fixed(View v, DCtl *dc, double dt, double idx, double idy
   if (v.ctl->done || nc >= dc->ncmax) return;
 
 // velocity at every cell (vlcty, common/mhd_class.hpp:59-65)
-__global__ void k_dvel(View v, const DCtl *dc, int nc)
+__device__ __forceinline__ void dvel_body(const View &v, int i, int j, int k)
 {
-  QAS_DSUB_GUARD();
-  QAS_CELL_INDEX();
   const long long c = cidx(v.g, i, j, k);
   const double iro = 1.0 / v.u[0][c];
   v.vx[c] = v.u[1][c] * iro;
   v.vy[c] = v.u[2][c] * iro;
   v.vz[c] = v.u[3][c] * iro;
 }
+static __global__ void k_dvel(View v, const DCtl *dc, int nc)
+{
+  QAS_DSUB_GUARD();
+  QAS_CELL_INDEX();
+  dvel_body(v, i, j, k);
+}
 
 // eta*J on the CT edges, mhd_ct_eres (common/mhd_func.c:78-106): in 2D with zoffset = 0 and
 // idz = 0 (dmhd2d_solve.cpp:46-54), in 3D with the real z stencils (dmhd3d_solve.cpp:48-57)
 template <int ODR>
-__global__ void k_eres(View v, const DCtl *dc, int nc, double eta0, double idx, double idy, double idz3 = 0.0)
+__device__ __forceinline__ void eres_body(const View &v, int i, int j, int k, double eta0, double idx, double idy,
+                                          double idz3)
 {
-  QAS_DSUB_GUARD();
-  QAS_CELL_INDEX();
   const Geo &g = v.g;
   if (i < 2 || i >= g.nx - 1 || j < 2 || j >= g.ny - 1) return;
   if (g.dim == 3 && (k < 2 || k >= g.nz - 1)) return;
@@ -105,6 +108,13 @@ __global__ void k_eres(View v, const DCtl *dc, int nc, double eta0, double idx, 
   v.ex[c] = 0.25 * (e + e + e + e) * jx;
   v.ey[c] = 0.25 * (e + e + e + e) * jy;
   v.ez[c] = 0.25 * (e + e + e + e) * jz;
+}
+template <int ODR>
+__global__ void k_eres(View v, const DCtl *dc, int nc, double eta0, double idx, double idy, double idz3 = 0.0)
+{
+  QAS_DSUB_GUARD();
+  QAS_CELL_INDEX();
+  eres_body<ODR>(v, i, j, k, eta0, idx, idy, idz3);
 }
 
 // viscous face flux at i-1/2 along stride xo with transverse strides yo, zo (0 for the
@@ -171,10 +181,9 @@ __device__ __forceinline__ void resist_flux(const double *by, const double *bz, 
 }
 
 template <int ODR>
-__global__ void k_dflux(View v, const DCtl *dc, int nc, double nu0, double idx, double idy, double idz3 = 0.0)
+__device__ __forceinline__ void dflux_body(const View &v, int i, int j, int k, double nu0, double idx, double idy,
+                                           double idz3)
 {
-  QAS_DSUB_GUARD();
-  QAS_CELL_INDEX();
   const Geo &g = v.g;
   if (i < 2 || i >= g.nx - 1 || j < 2 || j >= g.ny - 1) return;
   const bool d3 = g.dim == 3;
@@ -221,6 +230,13 @@ __global__ void k_dflux(View v, const DCtl *dc, int nc, double nu0, double idx, 
     v.f[2][7][c] = fenv + fenr;
   }
 }
+template <int ODR>
+__global__ void k_dflux(View v, const DCtl *dc, int nc, double nu0, double idx, double idy, double idz3 = 0.0)
+{
+  QAS_DSUB_GUARD();
+  QAS_CELL_INDEX();
+  dflux_body<ODR>(v, i, j, k, nu0, idx, idy, idz3);
+}
 
 // RK update of the 2D dsptv (dmhd2d_solve.cpp:107-146)
 template <int ODR>
@@ -253,10 +269,10 @@ __device__ __forceinline__ void dupdate2(const View &v, const DCtl *dc, int i, i
   }
   if (ci && cj) {
 #pragma unroll
-    for (int q = 0; q < 6; q++) v.u[cen[q]][c] = nv[q];
+    for (int q = 0; q < 6; q++) v.uo[cen[q]][c] = nv[q];
   }
-  if (cj) v.u[4][c] = nbx;
-  if (ci) v.u[5][c] = nby;
+  if (cj) v.uo[4][c] = nbx;
+  if (ci) v.uo[5][c] = nby;
 }
 
 // RK update of the 3D dsptv (dmhd3d_solve.cpp:114-167): mhd_updt3d on ro,mx,my,mz,en over the
@@ -298,11 +314,11 @@ __device__ __forceinline__ void dupdate3(const View &v, const DCtl *dc, int i, i
   }
   if (ci && cj && ck) {
 #pragma unroll
-    for (int q = 0; q < 5; q++) v.u[cen[q]][c] = nv[q];
+    for (int q = 0; q < 5; q++) v.uo[cen[q]][c] = nv[q];
   }
-  if (cj && ck) v.u[4][c] = nb[0];
-  if (ci && ck) v.u[5][c] = nb[1];
-  if (ci && cj) v.u[6][c] = nb[2];
+  if (cj && ck) v.uo[4][c] = nb[0];
+  if (ci && ck) v.uo[5][c] = nb[1];
+  if (ci && cj) v.uo[6][c] = nb[2];
 }
 
 template <int ODR>
@@ -324,7 +340,7 @@ __global__ void k_dupdate(View v, const DCtl *dc, int nc, double c0, double c1)
   }
 }
 
-__global__ void k_dbound(View v, const DCtl *dc, int nc)
+static __global__ void k_dbound(View v, const DCtl *dc, int nc)
 {
   QAS_DSUB_GUARD();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -335,7 +351,7 @@ __global__ void k_dbound(View v, const DCtl *dc, int nc)
 }
 
 // ut = u at the start of each dsptv call
-__global__ void k_dcopy(View v, const DCtl *dc, int nc)
+static __global__ void k_dcopy(View v, const DCtl *dc, int nc)
 {
   QAS_DSUB_GUARD();
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;

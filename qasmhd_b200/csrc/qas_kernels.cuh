@@ -298,7 +298,7 @@ __device__ __forceinline__ void dv_body(const View &v, int i, int j, int k)
     v.dv[a][c] = fac * raw;
   }
 }
-__global__ void k_dv(View v)
+static __global__ void k_dv(View v)
 {
   pdl_begin();
   if (v.ctl->done) return;
@@ -717,27 +717,6 @@ __device__ __forceinline__ void sweep_x_cell(const View &v, int i, int j, int k,
   if (lane >= 1 && have_cell && i >= 3) face_flux<RMN, 0>(v, c, l - 1, r);
 }
 
-// x sweep: 31 faces per warp over the flattened cells of all rows
-template <int ODR, int RMN, int PR>
-__global__ void __launch_bounds__(SWB, QAS_SWEEP_MINB_OF(RMN)) k_sweep_x(const __grid_constant__ View v, long long nwarps)
-{
-  pdl_begin();
-  if (v.ctl->done) return;
-  __shared__ double sm[SLOTS * SLP];
-  const Geo &g = v.g;
-  const int lane = threadIdx.x & 31;
-  const long long w = (long long)blockIdx.x * (SWB / 32) + (threadIdx.x >> 5);
-  if (w >= nwarps) return;  // the whole warp leaves together
-  const long long ncell = g.nx - 4;
-  const long long total = ncell * g.ny * g.nz;
-  long long t = w * 31 + lane;
-  const bool have_cell = t < total;
-  if (!have_cell) t = total - 1;  // a valid cell, computed and discarded (keeps the warp converged)
-  const long long row = t / ncell;
-  const int i = 2 + (int)(t - row * ncell);
-  sweep_x_cell<ODR, RMN, PR>(v, i, (int)(row % g.ny), (int)(row / g.ny), lane, have_cell, sm);
-}
-
 __device__ __forceinline__ void prefetch_l1(const double *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
 // one block's 32 columns of a y / z sweep: the faces p in [p0, p1) along A of the columns through
@@ -781,22 +760,58 @@ __device__ __forceinline__ void sweep_columns(const View &v, int i, int o, bool 
   }
 }
 
-// y / z sweep: 32 columns per block, marching over `seg` faces along A
-template <int ODR, int RMN, int A, int PR>
-__global__ void __launch_bounds__(SWB, QAS_SWEEP_MINB_OF(RMN)) k_sweep_m(const __grid_constant__ View v, int seg)
+// the blocks of a sweep launch: first those of the z faces, then y (bq[A - 1] blocks each, cols[A - 1]
+// column groups by segments of seg[A - 1] faces), last x (nwarps warps of 31 faces)
+struct SweepPlan {
+  unsigned bq[2], cols[2];
+  int seg[2];
+  long long nwarps;
+};
+
+// block `blk` of a sweep over the axes AX (bit a).  The y / z blocks march over `seg` faces of 32 columns;
+// an x warp takes 31 faces of the flattened cells of all rows.
+template <int ODR, int RMN, int PR, int AX>
+__device__ __forceinline__ void sweep_block(const View &v, const SweepPlan &pl, unsigned blk, double *sm)
 {
-  pdl_begin();
-  if (v.ctl->done) return;
   const Geo &g = v.g;
-  __shared__ double sm[SLOTS * SLP];
-  const int no = A == 1 ? g.nz : g.ny;  // extent of the other transverse axis
-  const long long cols = (long long)g.nx * no;
-  long long col = (long long)blockIdx.x * 32 + (threadIdx.x & 31);
-  const bool have = col < cols;
-  if (!have) col = cols - 1;
-  const int p0 = 3 + blockIdx.y * seg;
-  sweep_columns<ODR, RMN, A, PR>(v, (int)(col % g.nx), (int)(col / g.nx), have, p0, min(p0 + seg, g.n[A] - 2), sm);
+  const int lane = threadIdx.x & 31;
+  if ((AX & 6) != 0 && (AX == 2 || AX == 4 || blk < pl.bq[1] + pl.bq[0])) {
+    const bool z = AX == 4 || (AX != 2 && blk < pl.bq[1]);
+    if (AX == 7 && !z) blk -= pl.bq[1];
+    const int q = z ? 1 : 0, no = z ? g.ny : g.nz;
+    const unsigned s = blk / pl.cols[q];
+    const long long cols = (long long)g.nx * no;
+    long long col = (long long)(blk - s * pl.cols[q]) * 32 + lane;
+    const bool have = col < cols;
+    if (!have) col = cols - 1;
+    const int p0 = 3 + (int)s * pl.seg[q], p1 = min(p0 + pl.seg[q], g.n[1 + q] - 2);
+    const int i = (int)(col % g.nx), o = (int)(col / g.nx);
+    if constexpr ((AX & 4) != 0) {
+      if (z) sweep_columns<ODR, RMN, 2, PR>(v, i, o, have, p0, p1, sm);
+    }
+    if constexpr ((AX & 2) != 0) {
+      if (!z) sweep_columns<ODR, RMN, 1, PR>(v, i, o, have, p0, p1, sm);
+    }
+    return;
+  }
+  if constexpr ((AX & 1) == 0) return;
+  blk -= pl.bq[1] + pl.bq[0];
+  const long long w = (long long)blk * (SWB / 32) + (threadIdx.x >> 5);
+  if (w >= pl.nwarps) return;  // the whole warp leaves together
+  const long long ncell = g.nx - 4;
+  const long long total = ncell * g.ny * g.nz;
+  long long t = w * 31 + lane;
+  const bool have_cell = t < total;
+  if (!have_cell) t = total - 1;  // a valid cell, computed and discarded (keeps the warp converged)
+  const long long row = t / ncell;
+  const int i = 2 + (int)(t - row * ncell);
+  sweep_x_cell<ODR, RMN, PR>(v, i, (int)(row % g.ny), (int)(row / g.ny), lane, have_cell, sm);
 }
+
+// the sweep kernel (qas_sweep.cu) of an order (2 or 4), solver, reconstruction form (any: all three, else
+// characteristic or primitive) and set of axes (one, or 7 at the 2nd order)
+using SweepFn = void (*)(const View, const SweepPlan);
+SweepFn sweep_kernel(int odr, int rmn, bool any, int ax);
 
 // ---------------------------------------------------------------------------
 // corner EMFs (mhd2d_solve.cpp:201-232, :308-339; mhd3d_solve.cpp:259-328,
@@ -1135,14 +1150,14 @@ __device__ __forceinline__ void begin_body(const View &v, int check_tim)
   c->dtd[2] = v.g.dim >= 3 ? c->dt / v.dz : 0.0;
   c->vmax_bits = (unsigned long long)__double_as_longlong(1.0);  // for the setdt after this step
 }
-__global__ void k_begin_step(View v, int check_tim)
+static __global__ void k_begin_step(View v, int check_tim)
 {
   pdl_begin();
   begin_body(v, check_tim);
 }
 
 // dt/dx etc. for a host-supplied dt (a call of its own: qas_step), the stop flag taken back
-__global__ void k_set_dt(View v, double dt)
+static __global__ void k_set_dt(View v, double dt)
 {
   pdl_begin();
   Ctl *c = v.ctl;
@@ -1204,7 +1219,7 @@ __device__ __forceinline__ double vmax_cell(const View &v, int i, int j, int k)
 
 // max over the interior of |v| + c_f with B from the 2nd-order face average
 // (mhd2d_class.cpp:17-26); NaN never wins, as with `if (vtmp > vmax)`.
-__global__ void k_vmax(View v)
+static __global__ void k_vmax(View v)
 {
   pdl_begin();
   if (v.ctl->done) return;
@@ -1255,14 +1270,14 @@ __device__ __forceinline__ void setdt_body(const View &v, double cfl, double dr,
     c->first = 0;
   }
 }
-__global__ void k_setdt(View v, double cfl, double dr, int rule, double dtrec, int nout)
+static __global__ void k_setdt(View v, double cfl, double dr, int rule, double dtrec, int nout)
 {
   pdl_begin();
   setdt_body(v, cfl, dr, rule, dtrec, nout);
 }
 
 // k_vmax and k_setdt in one launch: blocks stride over the interior, the last one to finish sets dt
-__global__ void k_vmax_dt(View v, double cfl, double dr, int rule, double dtrec, int nout)
+static __global__ void k_vmax_dt(View v, double cfl, double dr, int rule, double dtrec, int nout)
 {
   pdl_begin();
   if (v.ctl->done) return;
@@ -1295,7 +1310,6 @@ __global__ void k_vmax_dt(View v, double cfl, double dr, int rule, double dtrec,
     setdt_body(v, cfl, dr, rule, dtrec, nout);
   }
 }
-
 // |div B| with df1[ODR-1] over the interior; max by bit pattern of non-negative doubles
 template <int ODR>
 __global__ void k_divb(View v, unsigned long long *out)
@@ -1321,7 +1335,7 @@ __global__ void k_divb(View v, unsigned long long *out)
 }
 
 // FP64 throughput probe: 8 independent DFMA chains per thread (2 flops each)
-__global__ void k_fp64_peak(double *out, int iters, double a, double b)
+static __global__ void k_fp64_peak(double *out, int iters, double a, double b)
 {
   double x0 = threadIdx.x * 1e-9, x1 = x0 + 1.0, x2 = x0 + 2.0, x3 = x0 + 3.0;
   double x4 = x0 + 4.0, x5 = x0 + 5.0, x6 = x0 + 6.0, x7 = x0 + 7.0;

@@ -18,10 +18,11 @@ import tempfile
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libqas.so")
-SOURCES = ["qas_api.cu", "qas_sweep.cu"]
+SOURCES = ["qas_api.cu", "qas_sweep.cu", "qas_stage1d.cu"]
 HEADERS = ["qas_device.cuh", "qas_kernels.cuh", "qas_dissip.cuh", "qas_batch.cuh", "qas_batch_api.inc",
            "qas_adjoint.cuh", "qas_adjoint_kernels.cuh", "qas_adjoint_api.inc", "qas_noalloc.inc",
-           "qas_io.inc", "qas_tma.cuh", "qas_dd.inc", "qas_hall.cuh", "qas_pipe.cuh", "qas_pipe.inc"]
+           "qas_io.inc", "qas_tma.cuh", "qas_dd.inc", "qas_hall.cuh", "qas_pipe.cuh", "qas_pipe.inc",
+           "qas_stage1d.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -24,7 +24,9 @@
 #include "qas_tma.cuh"
 #include "qas_hall.cuh"
 #include "qas_pipe.cuh"
+#include "qas_stage1d.cuh"
 #ifndef QAS_SEPARATE_UNITS  // the build compiles these side by side
+#include "qas_stage1d.cu"
 #include "qas_sweep.cu"
 #endif
 
@@ -920,10 +922,47 @@ bool hall_active(const qas_ctx *c) { return c->hall && c->hall_di != 0; }
 // the state in between (gravity's setdt rounds the energy, Hall sub-cycles start from a fill)
 bool ghosts_kept(const qas_ctx *c) { return !c->view.phi && !hall_active(c); }
 
+// 1D steps in one kernel a stage (qas_stage1d.cuh): the orders it is built for, at least two stages (a
+// block's neighbours read its cells while it writes), no Hall form, no form asked for or timed apart.
+// Brio-Wu 1024: 62.7 us a step in 17 launches, 22.6 us in 3.
+bool one_kernel_stages(const qas_ctx *c)
+{
+  return c->geo.dim == 1 && (c->scheme.odr == 4 || c->scheme.odr == 2) && c->scheme.rk >= 2 &&
+         c->scheme.char_mode != 2 && !c->hall && !c->fused_set && !c->prof;
+}
+// one exec_ iteration of such a context, its counters included: u -> u0 arrays -> the (unused) face-state
+// arrays -> u; bx never changes
+long long launch_step1(qas_ctx *c, int check_tim)
+{
+  const View &b = c->view;
+  const int R = c->scheme.rk;
+  const Stage1Fn fn = stage1_kernel(c->scheme.odr, c->scheme.rmn);
+  const unsigned nb = (unsigned)((c->grid.nxm + S1_TC - 1) / S1_TC);
+  for (int rk = 0; rk < R; rk++) {
+    double c0, c1;
+    rk_factors(R, rk, c0, c1);
+    View v = b;
+    for (int m = 0; m < 8; m++) {
+      if (m == 4) continue;
+      double *const w[2] = {b.u0[m], m < 7 ? b.vl[m] : b.vr[0]};
+      v.u[m] = rk == 0 ? b.u[m] : w[rk - 1];
+      v.uo[m] = rk == R - 1 ? b.u[m] : w[rk];
+      v.u0[m] = b.u[m];
+    }
+    launch(c, fn, nb, S1_NT, v, c0, c1, check_tim, rk == R - 1 ? 1 : 0);
+  }
+  return R;
+}
+
 // fill: the ghost fill at the start of the step
 long long launch_exec_step(qas_ctx *c, const qas_run_opts &o, int n_after, bool fill = true)
 {
   long long nk = 0;
+  if (one_kernel_stages(c)) {
+    nk = launch_step1(c, o.stop_rule == 2 ? 0 : 1);
+    if (o.flg && (n_after % 2 == 0)) nk += launch_setdt(c, o.cfl, o.stop_rule, o.dtrec, o.nout, false);
+    return nk;
+  }
   QL(c, KID_BEGIN, launch(c, k_begin_step, 1, 1, c->view, o.stop_rule == 2 ? 0 : 1));
   if (fill) QL(c, KID_BOUND, launch(c, k_bound<BOUND_STAGE>, shell_grid(c->geo), BLK, c->view, 0));
   if (hall_active(c)) nk += launch_hall_subcycles(c, o.cfl);
@@ -1368,8 +1407,8 @@ qas_status qas_run(qas_ctx *c, const qas_run_opts *opts, qas_run_info *info)
   int n_host = n0;
   const int limit = o.max_steps > 0 ? o.max_steps : INT_MAX;
   int launched = 0;
-  const bool fill = !ghosts_kept(c);
-  if (!fill) {  // once for all steps of the call
+  const bool fill = !ghosts_kept(c), one = one_kernel_stages(c);
+  if (!fill && !one) {  // once for all steps of the call
     launch(c, k_bound<BOUND_START>, shell_grid(c->geo), BLK, c->view, o.stop_rule == 2 ? 0 : 1);
     c->launches++;
   }
@@ -1431,6 +1470,10 @@ qas_status qas_run(qas_ctx *c, const qas_run_opts *opts, qas_run_info *info)
       if ((s = read_ctl(c)) != QAS_OK) return s;
       if (c->h_ctl->done) break;
     }
+  }
+  if (one) {  // its stages leave the ghosts alone
+    launch(c, k_bound_end, shell_grid(c->geo), BLK, c->view, n0);
+    c->launches++;
   }
   return end_run(c, n0, info);
   QAS_API_CATCH

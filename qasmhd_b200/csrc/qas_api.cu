@@ -118,6 +118,8 @@ struct qas_ctx {
   long long graph_kernels = 0;
   long long launches = 0;
   bool capturing = false;
+  bool plain_edges = false;  // the graph being captured takes plain edges (launch)
+  cudaError_t capture_err = cudaSuccess;  // of a call inside the capture
   qas_status latched = QAS_OK;
   // thread-block tile (x,y,z extents, 128 threads) of every cell kernel, by kernel id
   dim3 tile[32];
@@ -293,10 +295,10 @@ namespace {
 
 enum Kid {
   KID_PRIM, KID_DV, KID_LR, KID_FLUX, KID_EMF, KID_UPDATE, KID_BOUND, KID_BEGIN, KID_VMAX, KID_SETDT,
-  KID_DVEL, KID_ERES, KID_DFLUX, KID_DUPDATE, KID_DBOUND, KID_DCOPY, KID_DSUB, KID_SWEEP, KID_COUNT
+  KID_ERES, KID_DFLUX, KID_DUPDATE, KID_DBOUND, KID_DCOPY, KID_DSUB, KID_SWEEP, KID_COUNT
 };
 const char *const KID_NAMES[KID_COUNT] = {"k_prim", "k_dv", "k_lr", "k_flux", "k_emf", "k_update", "k_bound",
-                                          "k_begin_step", "k_vmax", "k_setdt", "k_dvel", "k_eres", "k_dflux",
+                                          "k_begin_step", "k_vmax", "k_setdt", "k_eres", "k_dflux",
                                           "k_dupdate", "k_dbound", "k_dcopy", "k_dsub", "k_sweep"};
 
 void prof_mark(qas_ctx *c, int kid)
@@ -343,7 +345,7 @@ template <class... KArgs, class... Args>
 void launch(qas_ctx *c, void (*kern)(KArgs...), dim3 grid, dim3 block, Args... args)
 {
   cudaError_t e = cudaSuccess;
-  if (c->capturing && c->geo.nd < (1 << 17))
+  if (c->capturing && c->plain_edges)
     kern<<<grid, block, 0, c->stream>>>(args...);
   else
     pdl_launch(e, kern, grid, block, c->stream, args...);
@@ -794,55 +796,120 @@ long long launch_ideal(qas_ctx *c)
   return nk;
 }
 
+// sub-cycle nc; fill: the ghost fill before it (else they are as the last stage left them).  As in
+// launch_ideal, ut stays in the state's arrays until the last stage writes them.
 template <int ODR>
-long long dsptv_odr(qas_ctx *c, int nc, double nu0, double eta0)
+long long dsptv_odr(qas_ctx *c, int nc, double nu0, double eta0, bool fill)
 {
   const Geo &g = c->geo;
   const double idx = 1.0 / c->grid.dx, idy = 1.0 / c->grid.dy;
   const double idz = g.dim == 3 ? 1.0 / c->grid.dz : 0.0;
+  const int R = c->scheme.rk;
   long long nk = 0;
-  QL(c, KID_DBOUND, launch(c, k_dbound, shell_grid(g), BLK, c->view, c->d_dctl, nc));
-  QL(c, KID_DCOPY, launch(c, k_dcopy, (unsigned)((g.nd + 255) / 256), 256, c->view, c->d_dctl, nc));
-  nk += 2;
-  for (int rk = 0; rk < c->scheme.rk; rk++) {
-    double c0, c1;
-    rk_factors(c->scheme.rk, rk, c0, c1);
-    QL(c, KID_DVEL, launch(c, k_dvel, cells_grid(g), BLK, c->view, c->d_dctl, nc));
-    QL(c, KID_ERES, launch(c, k_eres<ODR>, cells_grid(g), BLK, c->view, c->d_dctl, nc, eta0, idx, idy, idz));
-    QL(c, KID_DFLUX,
-       launch(c, k_dflux<ODR>, cells_grid(g), BLK, c->view, c->d_dctl, nc, nu0, idx, idy, idz));
-    QL(c, KID_DUPDATE, launch(c, k_dupdate<ODR>, update_grid(g), BLK, c->view, c->d_dctl, nc, c0, c1));
+  if (fill) {
     QL(c, KID_DBOUND, launch(c, k_dbound, shell_grid(g), BLK, c->view, c->d_dctl, nc));
-    nk += 5;
+    nk++;
+  }
+  for (int rk = 0; rk < R; rk++) {
+    double c0, c1;
+    rk_factors(R, rk, c0, c1);
+    View v = c->view;
+    for (int m = 0; m < 8; m++) {
+      v.u[m] = rk == 0 ? c->view.u[m] : c->view.u0[m];
+      v.uo[m] = rk == R - 1 ? c->view.u[m] : c->view.u0[m];
+      v.u0[m] = c->view.u[m];
+    }
+    QL(c, KID_ERES, launch(c, k_eres<ODR>, cells_grid(g), BLK, v, c->d_dctl, nc, nu0, eta0, idx, idy, idz));
+    QL(c, KID_DFLUX, launch(c, k_dflux<ODR>, cells_grid(g), BLK, v, c->d_dctl, nc, nu0, idx, idy, idz));
+    QL(c, KID_DUPDATE, launch(c, k_dupdate<ODR>, update_grid(g), BLK, v, c->d_dctl, nc, c0, c1));
+    for (int m = 0; m < 8; m++) v.u[m] = v.uo[m];
+    QL(c, KID_DBOUND, launch(c, k_dbound, shell_grid(g), BLK, v, c->d_dctl, nc));
+    nk += 4;
   }
   return nk;
 }
 
-long long launch_dsptv(qas_ctx *c, int nc, double nu0, double eta0)
+long long launch_dsptv(qas_ctx *c, int nc, double nu0, double eta0, bool fill)
 {
   switch (c->scheme.odr) {
-    case 1: return dsptv_odr<1>(c, nc, nu0, eta0);
-    case 2: return dsptv_odr<2>(c, nc, nu0, eta0);
-    case 3: return dsptv_odr<3>(c, nc, nu0, eta0);
-    default: return dsptv_odr<4>(c, nc, nu0, eta0);
+    case 1: return dsptv_odr<1>(c, nc, nu0, eta0, fill);
+    case 2: return dsptv_odr<2>(c, nc, nu0, eta0, fill);
+    case 3: return dsptv_odr<3>(c, nc, nu0, eta0, fill);
+    default: return dsptv_odr<4>(c, nc, nu0, eta0, fill);
   }
 }
 
-// setdc + sub-cycled dsptv after ideal (dmhd2d_class.cpp:19-26, dmhd3d_class.cpp:20-28),
-// device-guarded
 bool diss_arrays(const qas_ctx *c) { return c->view.nu != nullptr; }
 
-long long launch_dissipate(qas_ctx *c, double nu0, double eta0)
+// the sub-cycles inside a captured step: a loop node whose body is one sub-cycle, run ncmax times (their
+// number is known on the device only).  `graph` is the step's graph, `loop` the node's handle, which
+// k_dsub_setup (captured before) and the body's last kernel set.
+cudaError_t capture_subcycles(qas_ctx *c, cudaGraph_t graph, cudaGraphConditionalHandle loop, double nu0, double eta0,
+                              long long &nk)
+{
+  cudaStreamCaptureStatus st;
+  const cudaGraphNode_t *deps = nullptr;
+  const cudaGraphEdgeData *edges = nullptr;
+  size_t nd = 0;
+  cudaError_t e = cudaStreamGetCaptureInfo_v3(c->stream, &st, nullptr, &graph, &deps, &edges, &nd);
+  if (e != cudaSuccess) return e;
+  cudaGraphNodeParams p = {};
+  p.type = cudaGraphNodeTypeConditional;
+  p.conditional.handle = loop;
+  p.conditional.type = cudaGraphCondTypeWhile;
+  p.conditional.size = 1;
+  cudaGraphNode_t node;
+  if ((e = cudaGraphAddNode(&node, graph, deps, nd, &p)) != cudaSuccess) return e;
+  cudaStream_t body = nullptr, outer = c->stream;
+  if ((e = cudaStreamCreateWithFlags(&body, cudaStreamNonBlocking)) != cudaSuccess) return e;
+  e = cudaStreamBeginCaptureToGraph(body, p.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                    cudaStreamCaptureModeThreadLocal);
+  if (e == cudaSuccess) {
+    c->stream = body;
+    nk += launch_dsptv(c, 0, nu0, eta0, false) + 1;
+    k_dsub_next<<<1, 1, 0, body>>>(c->d_dctl, loop);
+    c->stream = outer;
+    cudaGraph_t g = nullptr;
+    e = cudaStreamEndCapture(body, &g);
+  }
+  cudaStreamDestroy(body);
+  if (e != cudaSuccess) return e;
+  return cudaStreamUpdateCaptureDependencies(outer, &node, 1, cudaStreamSetCaptureDependencies);
+}
+
+// setdc + sub-cycled dsptv after ideal (dmhd2d_class.cpp:19-26, dmhd3d_class.cpp:20-28): issued eagerly,
+// NSUB_CAP sub-cycles that the device guards; in a graph, the loop above (KH 515x301, one sub-cycle of the eight:
+// 12 kernels instead of 136).  fill: the ghosts may not be filled yet
+long long launch_dissipate(qas_ctx *c, double nu0, double eta0, bool fill)
 {
   // setdc's maximum of max(2 nu, eta) over every cell: the installed profiles, else uniform
   const double dcmax0 = (2 * nu0 >= eta0) ? 2 * nu0 : eta0;
   const double dcmax = diss_arrays(c) ? c->diss_dcmax : (dcmax0 > 0.0 ? dcmax0 : 0.0);
   if (!(dcmax > 1e-15)) return 0;
   const double idz = c->grid.dim == 3 ? 1.0 / c->grid.dz : 0.0;
+  cudaGraphConditionalHandle loop = 0;
+  cudaGraph_t graph = nullptr;
+  if (c->capturing) {
+    cudaStreamCaptureStatus st;
+    const cudaGraphNode_t *deps = nullptr;
+    const cudaGraphEdgeData *edges = nullptr;
+    size_t nd = 0;
+    cudaError_t e = cudaStreamGetCaptureInfo_v3(c->stream, &st, nullptr, &graph, &deps, &edges, &nd);
+    if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&loop, graph, 0, cudaGraphCondAssignDefault);
+    if (e != cudaSuccess) {
+      c->capture_err = e;
+      return 0;
+    }
+  }
   QL(c, KID_DSUB, launch(c, k_dsub_setup, 1, 1, c->view, c->d_dctl, dcmax, c->dr, 1.0 / c->grid.dx,
-                                                       1.0 / c->grid.dy, NSUB_CAP, idz));
+                         1.0 / c->grid.dy, NSUB_CAP, idz, loop));
   long long nk = 1;
-  for (int nc = 0; nc < NSUB_CAP; nc++) nk += launch_dsptv(c, nc, nu0, eta0);
+  if (c->capturing) {
+    const cudaError_t e = capture_subcycles(c, graph, loop, nu0, eta0, nk);
+    if (e != cudaSuccess) c->capture_err = e;
+    return nk;
+  }
+  for (int nc = 0; nc < NSUB_CAP; nc++) nk += launch_dsptv(c, nc, nu0, eta0, fill && nc == 0);
   return nk;
 }
 
@@ -967,7 +1034,7 @@ long long launch_exec_step(qas_ctx *c, const qas_run_opts &o, int n_after, bool 
   if (fill) QL(c, KID_BOUND, launch(c, k_bound<BOUND_STAGE>, shell_grid(c->geo), BLK, c->view, 0));
   if (hall_active(c)) nk += launch_hall_subcycles(c, o.cfl);
   nk += 1 + (fill ? 1 : 0) + launch_ideal(c);
-  if (c->grid.dim >= 2 && (o.nu0 > 0.0 || o.eta0 > 0.0 || diss_arrays(c))) nk += launch_dissipate(c, o.nu0, o.eta0);
+  if (c->grid.dim >= 2 && (o.nu0 > 0.0 || o.eta0 > 0.0 || diss_arrays(c))) nk += launch_dissipate(c, o.nu0, o.eta0, false);
   if (o.flg && (n_after % 2 == 0)) nk += launch_setdt(c, o.cfl, o.stop_rule, o.dtrec, o.nout, false);
   return nk;
 }
@@ -1430,10 +1497,17 @@ qas_status qas_run(qas_ctx *c, const qas_run_opts *opts, qas_run_info *info)
       }
       cudaGraph_t gph;
       QAS_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+      const bool diss = o.nu0 > 0.0 || o.eta0 > 0.0 || diss_arrays(c);  // a loop node takes plain edges
+      c->plain_edges = c->geo.nd < (1 << 17) || diss;
+      c->capture_err = cudaSuccess;
       c->capturing = true;
       long long nk = launch_exec_step(c, o, 1, fill) + launch_exec_step(c, o, 2, fill);
       c->capturing = false;
       cudaError_t e = cudaStreamEndCapture(c->stream, &gph);
+      if (c->capture_err != cudaSuccess) {
+        if (e == cudaSuccess && gph) cudaGraphDestroy(gph);
+        return cuda_fail(c->capture_err, "graph capture");
+      }
       if (e != cudaSuccess) return cuda_fail(e, "graph capture");
       e = cudaGraphInstantiate(&c->graph, gph, 0);
       cudaGraphDestroy(gph);
@@ -1500,8 +1574,7 @@ qas_status qas_dsptv(qas_ctx *c, double dt, double nu0, double eta0)
     switch (c->scheme.odr) {
 #define QAS_DST(O)                                                                                        \
   case O:                                                                                                 \
-    launch(c, k_dvel, cells_grid(g), BLK, c->view, c->d_dctl, 0);                                  \
-    launch(c, k_eres<O>, cells_grid(g), BLK, c->view, c->d_dctl, 0, eta0, idx, idy, idz);          \
+    launch(c, k_eres<O>, cells_grid(g), BLK, c->view, c->d_dctl, 0, nu0, eta0, idx, idy, idz);     \
     launch(c, k_dflux<O>, cells_grid(g), BLK, c->view, c->d_dctl, 0, nu0, idx, idy, idz);          \
     launch(c, k_dupdate<O>, update_grid(g), BLK, c->view, c->d_dctl, 0, c0, c1);                   \
     launch(c, k_dbound, shell_grid(g), BLK, c->view, c->d_dctl, 0);                                \
@@ -1513,7 +1586,7 @@ qas_status qas_dsptv(qas_ctx *c, double dt, double nu0, double eta0)
       QAS_DST(4)
 #undef QAS_DST
     }
-    nk += 5;
+    nk += 4;
   }
   c->launches += nk;
   return check_launch(c);
@@ -1527,7 +1600,7 @@ qas_status qas_dissipate(qas_ctx *c, double dt, double nu0, double eta0)
   if (c->grid.dim < 2 || c->view.phi) return QAS_ERR_UNSUPPORTED;
   if (diss_arrays(c) && (nu0 != 0.0 || eta0 != 0.0)) return QAS_ERR_INVALID;
   launch(c, k_set_dt, 1, 1, c->view, dt);
-  c->launches += 1 + launch_dissipate(c, nu0, eta0);
+  c->launches += 1 + launch_dissipate(c, nu0, eta0, true);
   return check_launch(c);
   QAS_API_CATCH
 }

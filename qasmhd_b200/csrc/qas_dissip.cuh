@@ -12,14 +12,15 @@ namespace qas {
 // Extra device control for the sub-cycles: ncmax and dt/ncmax of the current step.
 struct DCtl {
   int ncmax;
-  int pad;
+  int nc;          // sub-cycles done (the graph's loop)
   double sdt;      // dt/ncmax
   double sdtd[3];  // sdt*idx, sdt*idy, sdt*idz (dtdx = dt*idx as in dsptv)
 };
 
 // setdc + ncmax = 1 + (int)(2*(dcmax*dt)/(dr*dr))
+// loop != 0: the handle of the graph's loop over the sub-cycles, entered when there are any
 static __global__ void k_dsub_setup(View v, DCtl *dc, double dcmax, double dr, double idx, double idy, int cap,
-                             double idz = 0.0)
+                                    double idz, cudaGraphConditionalHandle loop)
 {
   pdl_begin();
   if (v.ctl->done) return;
@@ -35,6 +36,14 @@ static __global__ void k_dsub_setup(View v, DCtl *dc, double dcmax, double dr, d
   dc->sdtd[0] = dc->sdt * idx;
   dc->sdtd[1] = dc->sdt * idy;
   dc->sdtd[2] = dc->sdt * idz;
+  dc->nc = 0;
+  if (loop && ncmax > 0) cudaGraphSetConditional(loop, 1);
+}
+// the end of the loop's body: once more while sub-cycles are left
+static __global__ void k_dsub_next(DCtl *dc, cudaGraphConditionalHandle loop)
+{
+  dc->nc += 1;
+  cudaGraphSetConditional(loop, dc->nc < dc->ncmax ? 1 : 0);
 }
 
 // host-supplied dt for one dsptv(dt) call
@@ -60,12 +69,6 @@ __device__ __forceinline__ void dvel_body(const View &v, int i, int j, int k)
   v.vx[c] = v.u[1][c] * iro;
   v.vy[c] = v.u[2][c] * iro;
   v.vz[c] = v.u[3][c] * iro;
-}
-static __global__ void k_dvel(View v, const DCtl *dc, int nc)
-{
-  QAS_DSUB_GUARD();
-  QAS_CELL_INDEX();
-  dvel_body(v, i, j, k);
 }
 
 // eta*J on the CT edges, mhd_ct_eres (common/mhd_func.c:78-106): in 2D with zoffset = 0 and
@@ -109,11 +112,13 @@ __device__ __forceinline__ void eres_body(const View &v, int i, int j, int k, do
   v.ey[c] = 0.25 * (e + e + e + e) * jy;
   v.ez[c] = 0.25 * (e + e + e + e) * jz;
 }
+// and, for the viscous fluxes, the velocity (not read without viscosity: their terms are zero)
 template <int ODR>
-__global__ void k_eres(View v, const DCtl *dc, int nc, double eta0, double idx, double idy, double idz3 = 0.0)
+__global__ void k_eres(View v, const DCtl *dc, int nc, double nu0, double eta0, double idx, double idy, double idz3)
 {
   QAS_DSUB_GUARD();
   QAS_CELL_INDEX();
+  if (v.nu || nu0 != 0.0) dvel_body(v, i, j, k);
   eres_body<ODR>(v, i, j, k, eta0, idx, idy, idz3);
 }
 
@@ -193,11 +198,12 @@ __device__ __forceinline__ void dflux_body(const View &v, int i, int j, int k, d
   const long long sz = d3 ? g.s[2] : 0;  // the absent axis has offset 0 and idz 0 in 2D
   const double idz = d3 ? idz3 : 0.0;
   const double *ro = v.u[0];
-  double fmx, fmy, fmz, fenv, fby, fbz, fenr;
+  double fmx = 0.0, fmy = 0.0, fmz = 0.0, fenv = 0.0, fby, fbz, fenr;
   // x face (dmhd2d_solve.cpp:70-82, dmhd3d_solve.cpp:72-84)
   const double *nua = v.nu;  // per-cell viscosity, or the uniform nu0
-  double rnu = nua ? 0.5 * (ro[c - 1] * nua[c - 1] + ro[c] * nua[c]) : 0.5 * (ro[c - 1] * nu0 + ro[c] * nu0);
-  visc_flux<ODR>(v.vx, v.vy, v.vz, c, rnu, idx, idy, idz, 1, sy, sz, fmx, fmy, fmz, fenv);
+  const bool visc = nua || nu0 != 0.0;
+  double rnu = !visc ? 0.0 : nua ? 0.5 * (ro[c - 1] * nua[c - 1] + ro[c] * nua[c]) : 0.5 * (ro[c - 1] * nu0 + ro[c] * nu0);
+  if (visc) visc_flux<ODR>(v.vx, v.vy, v.vz, c, rnu, idx, idy, idz, 1, sy, sz, fmx, fmy, fmz, fenv);
   resist_flux<ODR>(v.u[5], v.u[6], v.ey, v.ez, c, 1, sy, sz, fby, fbz, fenr);
   v.f[0][0][c] = 0.0 + 0.0;
   v.f[0][1][c] = fmx + 0.0;
@@ -207,8 +213,8 @@ __device__ __forceinline__ void dflux_body(const View &v, int i, int j, int k, d
   v.f[0][6][c] = 0.0 + fbz;
   v.f[0][7][c] = fenv + fenr;
   // y face (dmhd2d_solve.cpp:83-94, dmhd3d_solve.cpp:86-97)
-  rnu = nua ? 0.5 * (ro[c - sy] * nua[c - sy] + ro[c] * nua[c]) : 0.5 * (ro[c - sy] * nu0 + ro[c] * nu0);
-  visc_flux<ODR>(v.vy, v.vz, v.vx, c, rnu, idy, idz, idx, sy, sz, 1, fmx, fmy, fmz, fenv);
+  rnu = !visc ? 0.0 : nua ? 0.5 * (ro[c - sy] * nua[c - sy] + ro[c] * nua[c]) : 0.5 * (ro[c - sy] * nu0 + ro[c] * nu0);
+  if (visc) visc_flux<ODR>(v.vy, v.vz, v.vx, c, rnu, idy, idz, idx, sy, sz, 1, fmx, fmy, fmz, fenv);
   resist_flux<ODR>(v.u[6], v.u[4], v.ez, v.ex, c, sy, sz, 1, fby, fbz, fenr);
   v.f[1][0][c] = 0.0 + 0.0;
   v.f[1][2][c] = fmx + 0.0;
@@ -218,8 +224,8 @@ __device__ __forceinline__ void dflux_body(const View &v, int i, int j, int k, d
   v.f[1][4][c] = 0.0 + fbz;
   v.f[1][7][c] = fenv + fenr;
   if (d3) {  // z face (dmhd3d_solve.cpp:99-110)
-    rnu = nua ? 0.5 * (ro[c - sz] * nua[c - sz] + ro[c] * nua[c]) : 0.5 * (ro[c - sz] * nu0 + ro[c] * nu0);
-    visc_flux<ODR>(v.vz, v.vx, v.vy, c, rnu, idz, idx, idy, sz, 1, sy, fmx, fmy, fmz, fenv);
+    rnu = !visc ? 0.0 : nua ? 0.5 * (ro[c - sz] * nua[c - sz] + ro[c] * nua[c]) : 0.5 * (ro[c - sz] * nu0 + ro[c] * nu0);
+    if (visc) visc_flux<ODR>(v.vz, v.vx, v.vy, c, rnu, idz, idx, idy, sz, 1, sy, fmx, fmy, fmz, fenv);
     resist_flux<ODR>(v.u[4], v.u[5], v.ex, v.ey, c, sz, 1, sy, fby, fbz, fenr);
     v.f[2][0][c] = 0.0 + 0.0;
     v.f[2][3][c] = fmx + 0.0;
@@ -231,7 +237,7 @@ __device__ __forceinline__ void dflux_body(const View &v, int i, int j, int k, d
   }
 }
 template <int ODR>
-__global__ void k_dflux(View v, const DCtl *dc, int nc, double nu0, double idx, double idy, double idz3 = 0.0)
+__global__ void k_dflux(View v, const DCtl *dc, int nc, double nu0, double idx, double idy, double idz3)
 {
   QAS_DSUB_GUARD();
   QAS_CELL_INDEX();

@@ -156,6 +156,7 @@ __device__ __forceinline__ bool upd_region(const Geo &g, int m, int i, int j)
 // distinct but the compiler cannot prove it, and interleaving would serialise the loads)
 __global__ void k_a_update(AView a)
 {
+  pdl_begin();
   QAS_ADJ_CELL(a.g);
   double w[8], o[8];
 #pragma unroll
@@ -174,6 +175,7 @@ __global__ void k_a_update(AView a)
 // followed by the copy u0 = u (dsptv)
 __global__ void k_a_fold(AView a)
 {
+  pdl_begin();
   QAS_ADJ_CELL(a.g);
   double r[8];
 #pragma unroll
@@ -214,6 +216,7 @@ __device__ __forceinline__ bool corner_in(const Geo &g, int i, int j)
 
 __global__ void k_a_emf(AView a)
 {
+  pdl_begin();
   QAS_ADJ_CELL(a.g);
   const Geo &g = a.g;
   if (!corner_in(g, i, j)) {
@@ -423,12 +426,14 @@ __device__ __forceinline__ void a_lr_cell(const AView &a, int i, int j, long lon
 template <int A>
 __global__ void __launch_bounds__(128) k_a_flux(AView a)
 {
+  pdl_begin();
   QAS_ADJ_STRIPS(a_flux_cell<A>(a, i, j, t));
 }
 
 template <int A>
 __global__ void __launch_bounds__(128) k_a_lr(AView a)
 {
+  pdl_begin();
   QAS_ADJ_STRIPS(a_lr_cell<A>(a, i, j, t));
 }
 
@@ -438,6 +443,7 @@ __global__ void __launch_bounds__(128) k_a_lr(AView a)
 // ---------------------------------------------------------------------------
 __global__ void k_a_prim(AView a)
 {
+  pdl_begin();
   QAS_ADJ_CELL(a.g);
   const Geo &g = a.g;
   const long long sy = g.s[1];
@@ -527,6 +533,7 @@ __global__ void k_a_prim(AView a)
 // cell-centre B^T: cx(c) = fac * fcen(bx[s-1..s+2]) at the fill source s of c
 __global__ void k_a_cb(AView a)
 {
+  pdl_begin();
   QAS_ADJ_CELL(a.g);
   const Geo &g = a.g;
   const double w[4] = {-0.0625, 0.5625, 0.5625, -0.0625};  // fcen<4> weights of s-1, s, s+1, s+2
@@ -558,6 +565,7 @@ __device__ __forceinline__ bool dflux_in(const Geo &g, int i, int j)
 
 __global__ void k_d_flux(AView a)
 {
+  pdl_begin();
   QAS_ADJ_CELL(a.g);
   const Geo &g = a.g;
   if (!dflux_in(g, i, j)) {
@@ -626,6 +634,7 @@ __device__ __forceinline__ double bz0_yface(const AView &a, long long f)
 
 __global__ void k_d_emf(AView a, double eta, double idx, double idy)
 {
+  pdl_begin();
   QAS_ADJ_CELL(a.g);
   const Geo &g = a.g;
   if (!dflux_in(g, i, j)) {
@@ -664,6 +673,7 @@ __global__ void k_d_emf(AView a, double eta, double idx, double idy)
 
 __global__ void k_d_b(AView a, double eta, double idx, double idy)
 {
+  pdl_begin();
   QAS_ADJ_CELL(a.g);
   const Geo &g = a.g;
   const long long sy = g.s[1];
@@ -741,6 +751,7 @@ __global__ void k_d_b(AView a, double eta, double idx, double idy)
 // deterministic sum of the per-cell eta adjoint (one block)
 __global__ void k_a_sum(const double *x, long long n, double *out)
 {
+  pdl_begin();
   __shared__ double sh[1024];
   double s = 0.0;
   for (long long k = threadIdx.x; k < n; k += blockDim.x) s += x[k];

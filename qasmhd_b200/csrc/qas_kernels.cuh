@@ -18,12 +18,14 @@
 // Resident-block caps of the memory-bound kernels (0: no launch bound, the compiler's choice).
 // Measured on B200 (OT 1024^2 / KH 160^3 per launch): k_update at 16 blocks (32 registers, a
 // few spills) 0.0887 -> 0.0804 ms / 0.383 -> 0.328 ms, k_prim at 16 0.125 -> 0.113 ms in 3D;
-// k_emf is slower capped (0.230 -> 0.250 ms at 12), so it keeps the compiler's choice.
+// k_emf and k_update by 32-bit offsets: k_update 77 -> 74 us / 323 -> 309 us, k_emf at 10 blocks (48
+// registers) 31.2 -> 29.7 us / 237 -> 234 us (capped with 64-bit addresses it spilled and was slower;
+// k_prim and k_dv gained nothing from them).
 #ifndef QAS_PRIM_MINB
 #define QAS_PRIM_MINB 16
 #endif
 #ifndef QAS_EMF_MINB
-#define QAS_EMF_MINB 0
+#define QAS_EMF_MINB 10
 #endif
 #ifndef QAS_UPDATE_MINB
 #define QAS_UPDATE_MINB 16
@@ -796,16 +798,15 @@ __device__ __forceinline__ void sweep_block(const View &v, const SweepPlan &pl, 
   }
   if constexpr ((AX & 1) == 0) return;
   blk -= pl.bq[1] + pl.bq[0];
-  const long long w = (long long)blk * (SWB / 32) + (threadIdx.x >> 5);
+  const unsigned w = blk * (SWB / 32) + (threadIdx.x >> 5);
   if (w >= pl.nwarps) return;  // the whole warp leaves together
-  const long long ncell = g.nx - 4;
-  const long long total = ncell * g.ny * g.nz;
-  long long t = w * 31 + lane;
+  const unsigned ncell = g.nx - 4;
+  const unsigned total = ncell * g.ny * g.nz;
+  unsigned t = w * 31 + lane;
   const bool have_cell = t < total;
   if (!have_cell) t = total - 1;  // a valid cell, computed and discarded (keeps the warp converged)
-  const long long row = t / ncell;
-  const int i = 2 + (int)(t - row * ncell);
-  sweep_x_cell<ODR, RMN, PR>(v, i, (int)(row % g.ny), (int)(row / g.ny), lane, have_cell, sm);
+  const unsigned row = t / ncell, k = row / g.ny;
+  sweep_x_cell<ODR, RMN, PR>(v, 2 + (t - row * ncell), row - k * g.ny, k, lane, have_cell, sm);
 }
 
 // the sweep kernel (qas_sweep.cu) of an order (2 or 4), solver, reconstruction form (any: all three, else
@@ -818,40 +819,43 @@ SweepFn sweep_kernel(int odr, int rmn, bool any, int ax);
 // :423-492, :587-656) with the CUCT weight (mhd_func.c:56-76) computed here.
 // ---------------------------------------------------------------------------
 template <int ODR>
-__device__ __forceinline__ double emf_term(const double *up, const double *cen, long long c, long long s, double sgn,
+__device__ __forceinline__ double emf_term(const double *up, const double *cen, unsigned c, unsigned s, double sgn,
                                            double wgt)
 {
   double a[5], b[5];
 #pragma unroll
   for (int m = 0; m < 5; m++) {
-    a[m] = up[c + (m - 3) * s];
-    b[m] = up[c + (m - 2) * s];
+    a[m] = *at(up, c + (m - 3) * s);
+    b[m] = *at(up, c + (m - 2) * s);
   }
   const double l0 = lin_left<ODR>(a), r0 = lin_right<ODR>(b);
 #pragma unroll
   for (int m = 0; m < 5; m++) {
-    a[m] = cen[c + (m - 3) * s];
-    b[m] = cen[c + (m - 2) * s];
+    a[m] = *at(cen, c + (m - 3) * s);
+    b[m] = *at(cen, c + (m - 2) * s);
   }
   const double l1 = lin_left<ODR>(a), r1 = lin_right<ODR>(b);
   return sgn * ((l0 + r0) + wgt * (l1 + r1));
 }
 
 __device__ __forceinline__ double cuct_at(const View &v, const double *va, const double *vb, const double *ba,
-                                          const double *bb, long long c, long long oa, long long ob)
+                                          const double *bb, unsigned c, unsigned oa, unsigned ob)
 {
   if (!v.ctw) return 0.5;
   const double *ro = v.u[0];
-  return cuct_weight(ro[c - oa - ob], ro[c - ob], ro[c - oa], ro[c], va[c - oa - ob], va[c - ob], va[c - oa], va[c],
-                     vb[c - oa - ob], vb[c - ob], vb[c - oa], vb[c], ba[c - ob], ba[c], bb[c - oa], bb[c]);
+  const unsigned cab = c - oa - ob, ca = c - oa, cb = c - ob;
+  return cuct_weight(*at(ro, cab), *at(ro, cb), *at(ro, ca), *at(ro, c), *at(va, cab), *at(va, cb), *at(va, ca),
+                     *at(va, c), *at(vb, cab), *at(vb, cb), *at(vb, ca), *at(vb, c), *at(ba, cb), *at(ba, c),
+                     *at(bb, ca), *at(bb, c));
 }
 
 template <int ODR>
 __device__ __forceinline__ void emf_body(const View &v, int i, int j, int k)
 {
   const Geo &g = v.g;
-  const long long c = cidx(g, i, j, k);
-  const long long sx = 1, sy = g.s[1], sz = g.s[2];
+  // 32-bit byte offsets
+  const unsigned c = 8u * (unsigned)cidx(g, i, j, k);
+  const unsigned sx = 8, sy = 8u * (unsigned)g.s[1], sz = 8u * (unsigned)g.s[2];
   const bool ii = i >= 3 && i < g.nx - 2, jj = j >= 3 && j < g.ny - 2;
   if (g.dim == 2) {
     if (ii && jj) {
@@ -859,7 +863,7 @@ __device__ __forceinline__ void emf_body(const View &v, int i, int j, int k)
       double ez = 0.0;
       ez += emf_term<ODR>(v.f[0][5], v.fc[0][0], c, sy, -0.5, (1.0 - ct));
       ez += emf_term<ODR>(v.f[1][4], v.fc[1][1], c, sx, +0.5, ct);
-      v.ez[c] = ez;
+      *at(v.ez, c) = ez;
     }
     return;
   }
@@ -869,21 +873,21 @@ __device__ __forceinline__ void emf_body(const View &v, int i, int j, int k)
     double ez = 0.0;
     ez += emf_term<ODR>(v.f[0][5], v.fc[0][0], c, sy, -0.5, (1.0 - ct0));
     ez += emf_term<ODR>(v.f[1][4], v.fc[1][1], c, sx, +0.5, ct0);
-    v.ez[c] = ez;
+    *at(v.ez, c) = ez;
   }
   if (ii && kk) {
     const double ct2 = cuct_at(v, v.vz, v.vx, v.u[6], v.u[4], c, sz, sx);
     double ey = 0.0;
     ey += emf_term<ODR>(v.f[0][6], v.fc[0][1], c, sz, +0.5, ct2);
     ey += emf_term<ODR>(v.f[2][4], v.fc[2][0], c, sx, -0.5, (1.0 - ct2));
-    v.ey[c] = ey;
+    *at(v.ey, c) = ey;
   }
   if (jj && kk) {
     const double ct1 = cuct_at(v, v.vy, v.vz, v.u[5], v.u[6], c, sy, sz);
     double ex = 0.0;
     ex += emf_term<ODR>(v.f[1][6], v.fc[1][0], c, sz, -0.5, (1.0 - ct1));
     ex += emf_term<ODR>(v.f[2][5], v.fc[2][1], c, sy, +0.5, ct1);
-    v.ex[c] = ex;
+    *at(v.ex, c) = ex;
   }
 }
 template <int ODR>
@@ -904,6 +908,12 @@ __device__ __forceinline__ double d4(const double *p, long long c, long long s)
 {
   return dfc<ODR>(p[c - s], p[c], p[c + s], p[c + 2 * s]);
 }
+// the same by byte offsets
+template <int ODR>
+__device__ __forceinline__ double d4_at(const double *p, unsigned c, unsigned s)
+{
+  return dfc<ODR>(*at(p, c - s), *at(p, c), *at(p, c + s), *at(p, c + 2 * s));
+}
 
 // update cell (i,j,k), i in [GH, nx-GH] etc.: the extra face of the staggered fields included.
 // The stage input is read from v.u, the new values go to v.uo
@@ -914,12 +924,12 @@ __device__ __forceinline__ void update_body(const View &v, int i, int j, int k, 
   // in the first stage (c0 = 0) ut is the stage input itself: not read a second time
   double *const *const ut = c0 == 0.0 ? v.u : v.u0;
   const Geo &g = v.g;
-  const long long c = cidx(g, i, j, k);
+  const unsigned c = 8u * (unsigned)cidx(g, i, j, k);  // 32-bit byte offsets
   const double dtdx = v.ctl->dtd[0], dtdy = v.ctl->dtd[1], dtdz = v.ctl->dtd[2];
   const bool ci = i < g.nx - GH;
   const bool cj = g.dim < 2 || j < g.ny - GH;
   const bool ck = g.dim < 3 || k < g.nz - GH;
-  const long long sy = g.s[1], sz = g.s[2];
+  const unsigned sy = 8u * (unsigned)g.s[1], sz = 8u * (unsigned)g.s[2];
   // every new value is formed before the first store (the compiler cannot prove that the
   // state and flux arrays do not alias, and interleaved stores would serialise the loads)
   double nv[8];
@@ -933,64 +943,64 @@ __device__ __forceinline__ void update_body(const View &v, int i, int j, int k, 
       if (g.dim >= 2 && m == 5) continue;
       if (g.dim >= 3 && m == 6) continue;
       double du;
-      const double du0 = d4<ODR>(v.f[0][m], c, 1);
+      const double du0 = d4_at<ODR>(v.f[0][m], c, 8);
       if (g.dim == 1) {
         du = -dtdx * du0;
       } else {
-        const double du1 = d4<ODR>(v.f[1][m], c, sy);
+        const double du1 = d4_at<ODR>(v.f[1][m], c, sy);
         if (g.dim == 2) {
           du = (-dtdx * du0 - dtdy * du1);
         } else {
-          const double du2 = d4<ODR>(v.f[2][m], c, sz);
+          const double du2 = d4_at<ODR>(v.f[2][m], c, sz);
           du = (-dtdx * du0 - dtdy * du1 - dtdz * du2);
         }
       }
-      nv[m] = rk_combine(ui[m][c], ut[m][c], du, c0, c1);
+      nv[m] = rk_combine(*at(ui[m], c), *at(ut[m], c), du, c0, c1);
       wr[m] = true;
     }
     if (v.phi) {
       // work done by gravity on the momentum, with the updated density (2D/SERIAL/RTI/
       // mhd2d_solve.cpp:361-362, 3D/MPI/RTI/mhd3d_solve.cpp:679-681)
       const double *ph = v.phi;
-      nv[1] = nv[1] + -c1 * nv[0] * 0.5 * (ph[c + 1] - ph[c - 1]) * dtdx;
-      nv[2] = nv[2] + -c1 * nv[0] * 0.5 * (ph[c + sy] - ph[c - sy]) * dtdy;
-      if (g.dim == 3) nv[3] = nv[3] + -c1 * nv[0] * 0.5 * (ph[c + sz] - ph[c - sz]) * dtdz;
+      nv[1] = nv[1] + -c1 * nv[0] * 0.5 * (*at(ph, c + 8) - *at(ph, c - 8)) * dtdx;
+      nv[2] = nv[2] + -c1 * nv[0] * 0.5 * (*at(ph, c + sy) - *at(ph, c - sy)) * dtdy;
+      if (g.dim == 3) nv[3] = nv[3] + -c1 * nv[0] * 0.5 * (*at(ph, c + sz) - *at(ph, c - sz)) * dtdz;
     }
   }
   if (g.dim == 2) {
     if (cj) {  // bx on i in [GH, nx-GH]
-      const double du = d4<ODR>(v.ez, c, sy);
-      nv[4] = rk_combine(ui[4][c], ut[4][c], -(+dtdy) * du, c0, c1);
+      const double du = d4_at<ODR>(v.ez, c, sy);
+      nv[4] = rk_combine(*at(ui[4], c), *at(ut[4], c), -(+dtdy) * du, c0, c1);
       wr[4] = true;
     }
     if (ci && j <= g.ny - GH) {  // by on j in [GH, ny-GH]
-      const double du = d4<ODR>(v.ez, c, 1);
-      nv[5] = rk_combine(ui[5][c], ut[5][c], -(-dtdx) * du, c0, c1);
+      const double du = d4_at<ODR>(v.ez, c, 8);
+      nv[5] = rk_combine(*at(ui[5], c), *at(ut[5], c), -(-dtdx) * du, c0, c1);
       wr[5] = true;
     }
   } else if (g.dim == 3) {
     if (ck && cj) {
-      const double du0 = +d4<ODR>(v.ez, c, sy);
-      const double du1 = -d4<ODR>(v.ey, c, sz);
-      nv[4] = rk_combine(ui[4][c], ut[4][c], -dtdy * du0 - dtdz * du1, c0, c1);
+      const double du0 = +d4_at<ODR>(v.ez, c, sy);
+      const double du1 = -d4_at<ODR>(v.ey, c, sz);
+      nv[4] = rk_combine(*at(ui[4], c), *at(ut[4], c), -dtdy * du0 - dtdz * du1, c0, c1);
       wr[4] = true;
     }
     if (ck && ci) {
-      const double du0 = +d4<ODR>(v.ex, c, sz);
-      const double du1 = -d4<ODR>(v.ez, c, 1);
-      nv[5] = rk_combine(ui[5][c], ut[5][c], -dtdz * du0 - dtdx * du1, c0, c1);
+      const double du0 = +d4_at<ODR>(v.ex, c, sz);
+      const double du1 = -d4_at<ODR>(v.ez, c, 8);
+      nv[5] = rk_combine(*at(ui[5], c), *at(ut[5], c), -dtdz * du0 - dtdx * du1, c0, c1);
       wr[5] = true;
     }
     if (cj && ci) {
-      const double du0 = +d4<ODR>(v.ey, c, 1);
-      const double du1 = -d4<ODR>(v.ex, c, sy);
-      nv[6] = rk_combine(ui[6][c], ut[6][c], -dtdx * du0 - dtdy * du1, c0, c1);
+      const double du0 = +d4_at<ODR>(v.ey, c, 8);
+      const double du1 = -d4_at<ODR>(v.ex, c, sy);
+      nv[6] = rk_combine(*at(ui[6], c), *at(ut[6], c), -dtdx * du0 - dtdy * du1, c0, c1);
       wr[6] = true;
     }
   }
 #pragma unroll
   for (int m = 0; m < 8; m++)
-    if (wr[m]) v.uo[m][c] = nv[m];
+    if (wr[m]) *at(v.uo[m], c) = nv[m];
 }
 
 // offset of the update launch: threads start at the first interior cell
@@ -1282,13 +1292,11 @@ static __global__ void k_vmax_dt(View v, double cfl, double dr, int rule, double
   pdl_begin();
   if (v.ctl->done) return;
   const Geo &g = v.g;
-  const long long mx = g.nx - 2 * GH, my = g.dim >= 2 ? g.ny - 2 * GH : 1, mz = g.dim >= 3 ? g.nz - 2 * GH : 1;
+  const unsigned mx = g.nx - 2 * GH, my = g.dim >= 2 ? g.ny - 2 * GH : 1, mz = g.dim >= 3 ? g.nz - 2 * GH : 1;
   double best = 1.0;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < mx * my * mz;
-       t += (long long)gridDim.x * blockDim.x) {
-    const long long r = t / mx;
-    const double vt = vmax_cell(v, GH + (int)(t - r * mx), (g.dim >= 2 ? GH : 0) + (int)(r % my),
-                                (g.dim >= 3 ? GH : 0) + (int)(r / my));
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < mx * my * mz; t += gridDim.x * blockDim.x) {
+    const unsigned r = t / mx, q = r / my;
+    const double vt = vmax_cell(v, GH + (t - r * mx), (g.dim >= 2 ? GH : 0) + (r - q * my), (g.dim >= 3 ? GH : 0) + q);
     if (vt > best) best = vt;
   }
 #pragma unroll

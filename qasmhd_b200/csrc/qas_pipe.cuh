@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(128, QAS_FLUX_MLAU_MINB) kw_flux_mlau(View v, 
   flux_body<3, A>(v, i, j, k);
 }
 
-// fused face sweeps on a window (the default form in 3D, see k_sweep_x / k_sweep_m)
+// fused face sweeps on a window (as k_sweep, one kernel for each axis of the wave)
 // x sweep over the flattened cells of the rows of planes r
 template <int ODR, int RMN, int PR>
 __global__ void __launch_bounds__(SWB, QAS_SWEEP_MINB_OF(RMN)) kw_sweep_x(const __grid_constant__ View v, Rows2 r, long long nwarps)
@@ -120,18 +120,18 @@ __global__ void __launch_bounds__(SWB, QAS_SWEEP_MINB_OF(RMN)) kw_sweep_x(const 
   __shared__ double sm[SLOTS * SLP];
   const Geo &g = v.g;
   const int lane = threadIdx.x & 31;
-  const long long w = (long long)blockIdx.x * (SWB / 32) + (threadIdx.x >> 5);
+  const unsigned w = blockIdx.x * (SWB / 32) + (threadIdx.x >> 5);
   if (w >= nwarps) return;  // the whole warp leaves together
-  const long long ncell = g.nx - 4;
-  const long long per_plane = g.dim == 3 ? g.ny : 1;
-  const long long total = ncell * per_plane * (rows_len(r.a) + rows_len(r.b));
-  long long t = w * 31 + lane;
+  const unsigned ncell = g.nx - 4;
+  const unsigned per_plane = g.dim == 3 ? g.ny : 1;
+  const unsigned total = ncell * per_plane * (rows_len(r.a) + rows_len(r.b));
+  unsigned t = w * 31 + lane;
   const bool have_cell = t < total;
   if (!have_cell) t = total - 1;
-  const long long row = t / ncell;
-  const int i = 2 + (int)(t - row * ncell);
-  const int j = g.dim == 3 ? (int)(row % g.ny) : rows2_plane(r, (int)row);
-  const int k = g.dim == 3 ? rows2_plane(r, (int)(row / g.ny)) : 0;
+  const unsigned row = t / ncell, plane = row / per_plane;
+  const int i = 2 + (t - row * ncell);
+  const int j = g.dim == 3 ? (int)(row - plane * per_plane) : rows2_plane(r, (int)row);
+  const int k = g.dim == 3 ? rows2_plane(r, (int)plane) : 0;
   sweep_x_cell<ODR, RMN, PR>(v, i, j, k, lane, have_cell, sm);
 }
 

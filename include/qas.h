@@ -268,9 +268,9 @@ qas_status qas_set_gravity(qas_ctx *ctx, const double *phi_g);
 /* Tuning options (defaults are the measured best on B200).
  *   QAS_OPT_FUSED_SWEEP: 0 = reconstruction and Riemann flux of each direction in two
  *   kernels with the face states in HBM (default in 1D); 1 = one fused sweep kernel per
- *   direction, the face states kept on chip (default in 3D; 4th-order interpolation only,
- *   other orders keep the two kernels).  The 2D default fuses x, and y for the HLLD solvers and
- *   on small grids.
+ *   direction, the face states kept on chip (default in 3D; 2nd and 4th-order interpolation,
+ *   other orders keep the two kernels; at the 2nd order one launch for all directions).  The 2D
+ *   default at the 4th order fuses x, and y for the HLLD solvers and on small grids.
  *   QAS_OPT_LR_STAGING: 1 = the reconstruction stages its stencils in shared memory with
  *   TMA tensor copies (available for 2D/3D, 4th-order interpolation, even padded x extent;
  *   QAS_ERR_UNSUPPORTED otherwise); 0 = it reads them from global memory (default: measured
@@ -278,7 +278,8 @@ qas_status qas_set_gravity(qas_ctx *ctx, const double *phi_g);
  * All forms give bit-identical results. */
 #define QAS_OPT_FUSED_SWEEP 1
 #define QAS_OPT_LR_STAGING 2
-#define QAS_OPT_PIPE_ITEMS 3 /* windows of planes of qas_step_host's wave, 1..64 (default 32) */
+#define QAS_OPT_PIPE_ITEMS 3 /* windows of planes of qas_step_host's wave, 1..64 (default by the grid's size,
+                                at most 32) */
 #define QAS_OPT_PIPE_LANES 4 /* streams of qas_step_host's stages, 1..3 (default 3 when their work arrays
                                 fit); set before the first qas_step_host of the context */
 /* Failure-path hook for tests of the bounded waits: value >= 0 makes every CTA of the TMA-staged

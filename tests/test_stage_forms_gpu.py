@@ -146,3 +146,16 @@ def test_step_keeps_the_callers_ghosts(restatement):
     want = np.ascontiguousarray(p.state.copy())
     assert restatement.lib.qo_step(ctypes.byref(g), restatement._ptr(want), 1e-3) == 0
     assert_bitwise(out, want, "step without bound")
+
+
+@pytest.mark.parametrize("n", [(24, 21), (150, 300), (12, 10, 14), (44, 46, 45)])
+def test_host_step_windows_by_size(restatement, n):
+    """The host round trip with the windows its grid selects: one, two and several."""
+    d = dict(zip(("nym", "nzm"), n[1:]))
+    p = P.orszag_tang(n[0], **d) if len(n) == 2 else P.kelvin_helmholtz(3, n[0], mach=0.2, rmn=3, **d)
+    a = restatement.run(p, 3, mode=R.MODE_RUN)
+    with L.Context.from_problem(p) as ctx:
+        x = np.ascontiguousarray(p.state.copy())
+        for _ in range(3):
+            ctx.step_host(x, x, flg=p.flg, cfl=p.cfl)
+        assert_bitwise(x, a["state"], f"{n}")

@@ -90,6 +90,48 @@ static void pipe_free(qas_ctx *c);
 static qas_status pipe_set_items(qas_ctx *c, int value);
 static qas_status pipe_set_lanes(qas_ctx *c, int value);
 
+// Streams of a graph capture on which independent launches (the face sweeps of the axes) become parallel
+// branches: fork() after the launch they depend on, stream(i) for the branches beside the main one, join()
+// before the launch that needs them all.  Temporary: the captured graph keeps no stream or event.
+struct Branches {
+  static constexpr int N = 3;
+  cudaStream_t st[N] = {};
+  cudaEvent_t at = nullptr, end[N] = {};
+  cudaError_t err = cudaSuccess;
+  void check(cudaError_t e)
+  {
+    if (err == cudaSuccess) err = e;
+  }
+  Branches()
+  {
+    check(cudaEventCreateWithFlags(&at, cudaEventDisableTiming));
+    for (int i = 0; i < N; i++) {
+      check(cudaStreamCreateWithFlags(&st[i], cudaStreamNonBlocking));
+      check(cudaEventCreateWithFlags(&end[i], cudaEventDisableTiming));
+    }
+  }
+  ~Branches()
+  {
+    for (int i = 0; i < N; i++) {
+      if (st[i]) cudaStreamDestroy(st[i]);
+      if (end[i]) cudaEventDestroy(end[i]);
+    }
+    if (at) cudaEventDestroy(at);
+  }
+  void fork(cudaStream_t main, int n)
+  {
+    check(cudaEventRecord(at, main));
+    for (int i = 0; i < n; i++) check(cudaStreamWaitEvent(st[i], at, 0));
+  }
+  void join(cudaStream_t main, int n)
+  {
+    for (int i = 0; i < n; i++) {
+      check(cudaEventRecord(end[i], st[i]));
+      check(cudaStreamWaitEvent(main, end[i], 0));
+    }
+  }
+};
+
 struct qas_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -118,6 +160,8 @@ struct qas_ctx {
   long long graph_kernels = 0;
   long long launches = 0;
   bool capturing = false;
+  Branches *branch = nullptr;  // while capturing a graph whose face sweeps run side by side
+  bool plain_next = false;     // the launches of a branch and of a join: plain edges
   bool plain_edges = false;  // the graph being captured takes plain edges (launch)
   cudaError_t capture_err = cudaSuccess;  // of a call inside the capture
   qas_status latched = QAS_OK;
@@ -345,7 +389,7 @@ template <class... KArgs, class... Args>
 void launch(qas_ctx *c, void (*kern)(KArgs...), dim3 grid, dim3 block, Args... args)
 {
   cudaError_t e = cudaSuccess;
-  if (c->capturing && c->plain_edges)
+  if (c->capturing && (c->plain_edges || c->plain_next))
     kern<<<grid, block, 0, c->stream>>>(args...);
   else
     pdl_launch(e, kern, grid, block, c->stream, args...);
@@ -697,9 +741,7 @@ long long stage_rest(qas_ctx *c, double c0, double c1)
   // a profile run keeps the 2D stage's two kernels apart, to time each
   const bool split = !sweep_built(c) || (c->prof && g.dim == 2 && !c->fused_set);
   const unsigned axes = split ? 0u : c->fused & ((1u << g.dim) - 1u);
-  if (axes) nk += launch_sweep(c, axes);
-  for (int a = 0; a < g.dim; a++) {
-    if ((axes >> a) & 1) continue;
+  auto two_kernels = [&](int a) {
     launch_lr<ODR>(c, a);
     switch (c->scheme.rmn) {
       case 0: launch_flux<0>(c, a); break;
@@ -708,12 +750,37 @@ long long stage_rest(qas_ctx *c, double c0, double c1)
       default: launch_flux<3>(c, a); break;
     }
     nk += 2;
+  };
+  // at most one axis writes the face-state arrays: its launches and the sweeps of the others touch nothing in
+  // common and become branches of the captured step, which fills each launch's last wave and, on small grids,
+  // idle SMs.  One after the other / side by side, us a step: RT 128x512 188 / 183, OT 512x400 336 / 326, OT
+  // 1024^2 1173 / 1159, KH 117x75x93 1973 / 1879, KH 160^3 7952 / 7907
+  const bool branches = ODR == 4 && c->branch && g.dim >= 2 && (axes & 1u) && (g.dim == 2 || axes == 7u);
+  if (branches) {
+    cudaStream_t outer = c->stream;
+    c->branch->fork(outer, g.dim - 1);
+    nk += launch_sweep(c, axes & 1u);
+    c->plain_next = true;
+    for (int a = 1; a < g.dim; a++) {
+      c->stream = c->branch->st[a - 1];
+      if ((axes >> a) & 1)
+        nk += launch_sweep(c, 1u << a);
+      else
+        two_kernels(a);
+    }
+    c->stream = outer;
+    c->branch->join(outer, g.dim - 1);
+  } else {
+    if (axes) nk += launch_sweep(c, axes);
+    for (int a = 0; a < g.dim; a++)
+      if (!((axes >> a) & 1)) two_kernels(a);
   }
   nk += launch_crcte(c);  // 1D Hall driver with electron inertia (hmhd1d_solve.cpp:98-108)
   if (g.dim >= 2) {
     QL(c, KID_EMF, launch(c, k_emf<ODR>, cells_grid(g, c->tile[KID_EMF]), c->tile[KID_EMF], c->view));
     nk++;
   }
+  c->plain_next = false;
   QL(c, KID_UPDATE, launch(c, k_update<ODR>, update_grid(g, c->tile[KID_UPDATE]), c->tile[KID_UPDATE], c->view, c0, c1));
   View out = c->view;
   for (int m = 0; m < 8; m++) out.u[m] = out.uo[m];
@@ -1500,9 +1567,15 @@ qas_status qas_run(qas_ctx *c, const qas_run_opts *opts, qas_run_info *info)
       const bool diss = o.nu0 > 0.0 || o.eta0 > 0.0 || diss_arrays(c);  // a loop node takes plain edges
       c->plain_edges = c->geo.nd < (1 << 17) || diss;
       c->capture_err = cudaSuccess;
+      Branches side;
+      const bool fork = side.err == cudaSuccess;
+      if (side.err != cudaSuccess) cudaGetLastError();
+      c->branch = fork ? &side : nullptr;
       c->capturing = true;
       long long nk = launch_exec_step(c, o, 1, fill) + launch_exec_step(c, o, 2, fill);
       c->capturing = false;
+      c->branch = nullptr;
+      if (fork && c->capture_err == cudaSuccess) c->capture_err = side.err;
       cudaError_t e = cudaStreamEndCapture(c->stream, &gph);
       if (c->capture_err != cudaSuccess) {
         if (e == cudaSuccess && gph) cudaGraphDestroy(gph);

@@ -39,7 +39,7 @@ ALG_BYTES_PER_CELL_UPDATE = 512  # 8 FP64 fields: stage 1 reads u^n, writes; sta
 #   k_flux   reads the 7+7 face states, the face normal field, the induction states (2/4), vn
 #            and the shock detector (MLAU/LHLLD: 1 in 2D, 2 in 3D); writes 8 fluxes and the
 #            central induction fluxes (1 in 2D, 2 in 3D)
-#   k_sweep  (face states + flux of one axis in one kernel, the 3D default) reads the 7 stencil
+#   k_sweep  (face states + flux of one axis in one kernel) reads the 7 stencil
 #            fields, the centre and face normal fields and the shock detector (1 in 2D, 2 in 3D,
 #            MLAU/LHLLD); writes 7 fluxes and the central induction fluxes (1 in 2D, 2 in 3D):
 #            the face states never leave the SM
@@ -49,18 +49,18 @@ KERNEL_ARRAYS = {
     "k_sweep": {1: 8 + 7, 2: 9 + 1 + 7 + 1, 3: 9 + 2 + 7 + 2},
 }
 # FP64 work per cell, counted by ncu (dadd + dmul + dfma instructions, and flops with a dfma
-# counted 2): k_lr on the 2D Orszag-Tang 1024^2 workload (ODR=4; profiles/k_lr_ot2d_1024.md),
-# k_sweep (MLAU) on KH 128^3 (profiles/k_sweep_kh3d_256.md: 1588-1604 per direction)
-FP64_INSTR_PER_CELL = {"k_lr": 1054.0, "k_sweep": 1600.0}
-FP64_FLOPS_PER_CELL = {"k_lr": 1262.0, "k_sweep": 1923.0}
+# counted 2): k_lr on the 2D Orszag-Tang 1024^2 workload (ODR=4), k_sweep (MLAU) on KH 128^3
+# (1410-1432 per direction); profiles/shared_march_sweeps.md
+FP64_INSTR_PER_CELL = {"k_lr": 968.0, "k_sweep": 1424.0}
+FP64_FLOPS_PER_CELL = {"k_lr": 1304.0, "k_sweep": 1902.0}
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch of the dominant kernel, per
-# workload: k_lr (y faces) of OT 1024^2 (profiles/k_lr_ot2d_1024.md); for KH 3D the KH 128^3
-# captures (136^3 padded cells: k_lr x faces 200.12 + 314.29 MB; k_sweep the mean of its x, y, z
-# launches, 378.0 + 405.8 + 405.0 MB / 3) scaled by padded cells to 264^3 (traffic per cell is
+# workload: k_lr (y faces) of OT 1024^2; for KH 3D the KH 128^3 captures (136^3 padded cells: k_lr
+# x faces 200.12 + 314.29 MB; k_sweep the mean of its x, y, z launches, 376 + 369 + 366 MB / 3;
+# profiles/shared_march_sweeps.md) scaled by padded cells to 264^3 (traffic per cell is
 # size-independent: every array is streamed once, the 126 MB L2 holds no full array)
-KERNEL_TRAFFIC_PER_LAUNCH = {("k_lr", "ot2d_1024"): 76.70e6 + 92.25e6,
+KERNEL_TRAFFIC_PER_LAUNCH = {("k_lr", "ot2d_1024"): 78e6 + 115e6,
                              ("k_lr", "kh3d_256"): (200.12e6 + 314.29e6) * (264 / 136) ** 3,
-                             ("k_sweep", "kh3d_256"): (378.0e6 + 405.8e6 + 405.0e6) / 3 * (264 / 136) ** 3}
+                             ("k_sweep", "kh3d_256"): (376e6 + 369e6 + 366e6) / 3 * (264 / 136) ** 3}
 
 
 def parse():

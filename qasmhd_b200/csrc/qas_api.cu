@@ -157,6 +157,7 @@ struct qas_ctx {
   int graph_flg = -1, graph_rule = -1;
   double graph_cfl = 0.0, graph_nu0 = -1.0, graph_eta0 = -1.0, graph_dtrec = 0.0;
   int graph_nout = 0;
+  unsigned graph_form = 0;  // stage_form() of its steps
   long long graph_kernels = 0;
   long long launches = 0;
   bool capturing = false;
@@ -1064,6 +1065,9 @@ bool one_kernel_stages(const qas_ctx *c)
   return c->geo.dim == 1 && (c->scheme.odr == 4 || c->scheme.odr == 2) && c->scheme.rk >= 2 &&
          c->scheme.char_mode != 2 && !c->hall && !c->fused_set && !c->prof;
 }
+// everything that decides which kernels a step consists of and an option can change between two runs: a
+// graph captured in another form is not replayed (a one-kernel step leaves the ghosts to the run's end)
+unsigned stage_form(const qas_ctx *c) { return c->fused | (c->lr_tma ? 8u : 0u) | (one_kernel_stages(c) ? 16u : 0u); }
 // one exec_ iteration of such a context, its counters included: u -> u0 arrays -> the (unused) face-state
 // arrays -> u; bx never changes
 long long launch_step1(qas_ctx *c, int check_tim)
@@ -1556,7 +1560,7 @@ qas_status qas_run(qas_ctx *c, const qas_run_opts *opts, qas_run_info *info)
   if (want_graph && launched + 2 <= limit) {
     const bool stale = !c->graph || c->graph_flg != o.flg || c->graph_rule != o.stop_rule || c->graph_cfl != o.cfl ||
                        c->graph_nu0 != o.nu0 || c->graph_eta0 != o.eta0 || c->graph_dtrec != o.dtrec ||
-                       c->graph_nout != o.nout;
+                       c->graph_nout != o.nout || c->graph_form != stage_form(c);
     if (stale) {
       if (c->graph) {
         cudaGraphExecDestroy(c->graph);
@@ -1593,6 +1597,7 @@ qas_status qas_run(qas_ctx *c, const qas_run_opts *opts, qas_run_info *info)
       c->graph_eta0 = o.eta0;
       c->graph_dtrec = o.dtrec;
       c->graph_nout = o.nout;
+      c->graph_form = stage_form(c);
     }
   }
   const int chunk = 32;  // steps between host checks of the stop flag
@@ -1905,11 +1910,6 @@ qas_status qas_set_option(qas_ctx *c, int option, int value)
   if (!c) return QAS_ERR_INVALID;
   if (option == QAS_OPT_FUSED_SWEEP) {
     const unsigned f = value != 0 ? 7u : 0u;
-    if (f != c->fused && c->graph) {  // the captured graph holds the other form
-      cudaStreamSynchronize(c->stream);
-      cudaGraphExecDestroy(c->graph);
-      c->graph = nullptr;
-    }
     c->fused = f;
     c->fused_set = true;
     if (f) sweep_prepare(c);
@@ -1918,11 +1918,6 @@ qas_status qas_set_option(qas_ctx *c, int option, int value)
   if (option == QAS_OPT_LR_STAGING) {
     const bool t = value != 0;
     if (t && !c->lr_tma_ok) return QAS_ERR_UNSUPPORTED;
-    if (t != c->lr_tma && c->graph) {
-      cudaStreamSynchronize(c->stream);
-      cudaGraphExecDestroy(c->graph);
-      c->graph = nullptr;
-    }
     c->lr_tma = t;
     // the staged kernel is a reconstruction of its own: in 2D it takes the place of the fused axes too
     if (c->geo.dim == 2 && !c->fused_set) c->fused = t ? 0u : fused_axes(c);

@@ -1618,10 +1618,8 @@ qas_status qas_run(qas_ctx *c, const qas_run_opts *opts, qas_run_info *info)
       }
     }
     if ((s = check_launch(c)) != QAS_OK) return s;
-    if (o.stop_rule != 0) {
-      if ((s = read_ctl(c)) != QAS_OK) return s;
-      if (c->h_ctl->done) break;
-    }
+    // an error that the device latched is returned by end_run
+    if (o.stop_rule != 0 && (read_ctl(c) != QAS_OK || c->h_ctl->done)) break;
   }
   if (one) {  // its stages leave the ghosts alone
     launch(c, k_bound_end, shell_grid(c->geo), BLK, c->view, n0);

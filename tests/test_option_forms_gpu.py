@@ -1,4 +1,6 @@
-"""Options set between two runs of a context: the state, ghosts included, against the oracle."""
+"""Options set between two runs of a context: the state, ghosts included, against the oracle.  The ghosts after a
+run that ends in a device error."""
+import numpy as np
 import pytest
 
 from oracle import refcase as R
@@ -34,3 +36,21 @@ def test_option_between_runs(restatement, dim, value, option):
             n += steps
             want = restatement.run(p, n, mode=R.MODE_RUN)["state"]
             assert_bitwise(ctx.download(p.state.shape), want, f"{dim}d option {option} = {value_}, {n} steps")
+
+
+@pytest.mark.parametrize("stop_rule", [0, 1])
+def test_1d_ghosts_after_a_refused_state(stop_rule):
+    """A run that ends with a latched device error leaves the ghosts filled from its last state, wherever in the
+    call the error is found."""
+    p = _periodic(1)
+    p.state[7, :, :, 30] = 0.05  # a negative pressure
+    with L.Context.from_problem(p) as ctx:
+        ctx.upload(p.state)
+        with pytest.raises(L.QasError) as e:
+            ctx.run(max_steps=40, flg=p.flg, cfl=p.cfl, stop_rule=stop_rule, dtrec=100.0)
+        assert e.value.status == L.QAS_ERR_NONFINITE
+        out = ctx.download(p.state.shape)
+    n = p.nxm
+    assert not np.array_equal(out, p.state, equal_nan=True)
+    assert_bitwise(out[..., :4], out[..., n:n + 4], "lower ghosts")
+    assert_bitwise(out[..., n + 4:], out[..., 4:8], "upper ghosts")

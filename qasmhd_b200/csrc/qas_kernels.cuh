@@ -321,7 +321,10 @@ static __global__ void k_dv(View v)
 
 // stencil accessor of k_lr: field f of (ro, vn, vb, vc, cb, cc, pr) along axis A at point m
 // (0..4) of cell c; the field pointers are read from the kernel's View parameter at each use,
-// so no pointer stays live in registers
+// so no pointer stays live in registers.  Plain loads, here and in the sweeps: a launch that overlaps its
+// predecessor (pdl_begin) starts while that one still writes these fields, and the non-coherent path (__ldg)
+// asks for data that nobody writes during the kernel's life.  A step with plain / non-coherent loads, us: KH
+// 160^3 8075 / 8015, KH 117x75x93 1918 / 1907, OT 1024^2 1172 / 1174, KH 64^3 at the 2nd order 559 / 575.
 template <int A>
 struct LrStencil {
   const View &v;
@@ -343,9 +346,7 @@ struct LrStencil {
       default: return v.pr;
     }
   }
-  __device__ __forceinline__ double operator()(int f, int m) const { return __ldg(at(field(f), c + (m - 2) * s)); }
-  // plain load, for reads issued after the face-state stores (kept in order behind them)
-  __device__ __forceinline__ double late(int f, int m) const { return *at(field(f), c + (m - 2) * s); }
+  __device__ __forceinline__ double operator()(int f, int m) const { return *at(field(f), c + (m - 2) * s); }
 };
 
 // face_states of cell c along A by the reference's divisions, out of line: what the kernels call for
@@ -416,8 +417,8 @@ __device__ __forceinline__ void lr_cell(const View &v, long long c, long long s,
       double prod[5], vts[5];
 #pragma unroll
       for (int m = 0; m < 5; m++) {
-        prod[m] = st.late(4 + t, m) * st.late(1, m);  // bt * vn
-        vts[m] = st.late(2 + t, m);                   // vt
+        prod[m] = st(4 + t, m) * st(1, m);  // bt * vn
+        vts[m] = st(2 + t, m);              // vt
       }
       double fl0, fr0, fl1, fr1;
       lin_lr<ODR>(prod, fl0, fr0);
@@ -648,16 +649,16 @@ __device__ __forceinline__ void cell_states(const View &v, long long c, double *
   if ((PR <= 0 && v.recon == 1) || (PR < 0 && v.recon == 2)) {
     double vl[7], vr[7];
     if (PR < 0 && v.recon == 2)
-      face_states_athena<ODR>(st, __ldg(at(cn, st.c)), v.gam, vl, vr);
+      face_states_athena<ODR>(st, *at(cn, st.c), v.gam, vl, vr);
     else
       face_states_prim<ODR>(st, vl, vr);
 #pragma unroll
     for (int m = 0; m < 7; m++) store(m, vl[m], vr[m]);
   } else {
-    face_states_emit<ODR>(st, __ldg(at(cn, st.c)), v.gam, store);
+    face_states_emit<ODR>(st, *at(cn, st.c), v.gam, store);
   }
   if (g.dim >= 2) {
-    const double bfl = __ldg(at(v.u[4 + A], st.c + st.s)), bfr = __ldg(at(v.u[4 + A], st.c));
+    const double bfl = *at(v.u[4 + A], st.c + st.s), bfr = *at(v.u[4 + A], st.c);
 #pragma unroll
     for (int t = 0; t < 2; t++) {
       if (g.dim == 2 && ((A == 0 && t == 1) || (A == 1 && t == 0))) continue;
@@ -684,17 +685,17 @@ __device__ __forceinline__ void face_flux(const View &v, long long f, const doub
   const long long s = g.s[A];
   constexpr int B = (A + 1) % 3, C = (A + 2) % 3;
   const unsigned o = (unsigned)(8 * f), so = (unsigned)(8 * s);
-  const double bn = __ldg(at(v.u[4 + A], o));  // the reference's 0.5*(bn + bn)
+  const double bn = *at(v.u[4 + A], o);  // the reference's 0.5*(bn + bn)
   double dv0 = 0.0, dv1 = 0.0;
   if (RMN >= 2) {
     const double *vn = A == 0 ? v.vx : (A == 1 ? v.vy : v.vz);
-    dv0 = __ldg(at(vn, o)) - __ldg(at(vn, o - so));
+    dv0 = *at(vn, o) - *at(vn, o - so);
     if (g.dim == 2) {
       const double *dt = v.dv[A == 0 ? 1 : 0];
-      dv1 = qmin(__ldg(at(dt, o - so)), __ldg(at(dt, o)));
+      dv1 = qmin(*at(dt, o - so), *at(dt, o));
     } else if (g.dim == 3) {
       const double *d1 = v.dv[B], *d2 = v.dv[C];
-      dv1 = qmin(qmin(__ldg(at(d1, o - so)), __ldg(at(d1, o))), qmin(__ldg(at(d2, o - so)), __ldg(at(d2, o))));
+      dv1 = qmin(qmin(*at(d1, o - so), *at(d1, o)), qmin(*at(d2, o - so), *at(d2, o)));
     }
   }
   double L[7], R[7];

@@ -113,7 +113,6 @@ struct SmemStencil {
     if (q >= R) q -= R;
     return ring[(q * 7 + f) * PD + idx];
   }
-  __device__ __forceinline__ double late(int f, int m) const { return (*this)(f, m); }
 };
 
 // dynamic shared memory of one configuration: ring slots x 7 fields x PD doubles + barriers
@@ -194,7 +193,7 @@ __global__ void __launch_bounds__(TX *TR, 5) k_lr_tma(const __grid_constant__ Vi
         const int j = MA == 1 ? m : rr, k = MA == 1 ? rr : m;
         const long long c = cidx(g, i, j, k);
         const SmemStencil<S::XS, S::PD, S::R> st{lr_ring, lrow * S::BX + lx, (int)((gbase + s) % S::R)};
-        lr_cell<ODR, A>(v, c, sA, st, __ldg(cn + c));
+        lr_cell<ODR, A>(v, c, sA, st, cn[c]);
       }
       if (__syncthreads_or(timeout)) {
         if (tid == 0) {

@@ -396,6 +396,13 @@ void launch(qas_ctx *c, void (*kern)(KArgs...), dim3 grid, dim3 block, Args... a
     pdl_launch(e, kern, grid, block, c->stream, args...);
 }
 
+// one whose kernel reads through the non-coherent path: without overlap
+template <class... KArgs, class... Args>
+void launch_plain(qas_ctx *c, void (*kern)(KArgs...), dim3 grid, dim3 block, Args... args)
+{
+  kern<<<grid, block, 0, c->stream>>>(args...);
+}
+
 // launch `expr` (one kernel) with optional event timing
 #define QL(c, kid, ...)                    \
   do {                                     \
@@ -570,9 +577,9 @@ void launch_lr(qas_ctx *c, int a)
     return;
   }
   if (c->view.recon == 2) {
-    if (a == 0) QL(c, KID_LR, launch(c, k_lr<ODR, 0, 2>, grid, blk, c->view));
-    if (a == 1) QL(c, KID_LR, launch(c, k_lr<ODR, 1, 2>, grid, blk, c->view));
-    if (a == 2) QL(c, KID_LR, launch(c, k_lr<ODR, 2, 2>, grid, blk, c->view));
+    if (a == 0) QL(c, KID_LR, launch_plain(c, k_lr<ODR, 0, 2>, grid, blk, c->view));
+    if (a == 1) QL(c, KID_LR, launch_plain(c, k_lr<ODR, 1, 2>, grid, blk, c->view));
+    if (a == 2) QL(c, KID_LR, launch_plain(c, k_lr<ODR, 2, 2>, grid, blk, c->view));
     return;
   }
   if (a == 0) QL(c, KID_LR, launch(c, k_lr<ODR, 0>, grid, blk, c->view));
@@ -683,7 +690,10 @@ long long launch_sweep(qas_ctx *c, unsigned axes)
     if (!ax || (nk && c->scheme.odr == 2)) continue;
     SweepPlan pl;
     const unsigned nb = sweep_plan(c, ax, pl);
-    QL(c, KID_SWEEP, launch(c, sweep_fn(c, a), nb, SWB, c->view, pl));
+    if (c->scheme.char_mode == 2)
+      QL(c, KID_SWEEP, launch_plain(c, sweep_fn(c, a), nb, SWB, c->view, pl));
+    else
+      QL(c, KID_SWEEP, launch(c, sweep_fn(c, a), nb, SWB, c->view, pl));
     nk++;
   }
   return nk;

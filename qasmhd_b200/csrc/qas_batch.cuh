@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(128, QAS_BATCH_LR_MINB) kb_lr(const View *__re
   QAS_BATCH_BLOCKS(map)
   if (QAS_BATCH_CELL_OK) {
     const int pos = A == 0 ? ti : (A == 1 ? tj : tk);
-    if (pos >= 2 && pos < v.g.n[A] - 2) lr_body<ODR, A, PR>(v, ti, tj, tk);
+    if (pos >= 2 && pos < v.g.n[A] - 2) lr_body<ODR, A, PR, true>(v, ti, tj, tk);
   }
   QAS_BATCH_END
 }
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(SWB, QAS_SWEEP_MINB_OF(RMN)) kb_sweep(const Vi
   const int2 b = blk[blockIdx.x];
   const View &v = views[b.x];
   if (v.ctl->done) return;
-  sweep_block<4, RMN, 0, 1 << A>(v, plans[b.x], (unsigned)b.y, sm);
+  sweep_block<4, RMN, 0, 1 << A, true>(v, plans[b.x], (unsigned)b.y, sm);
 }
 
 template <int ODR>

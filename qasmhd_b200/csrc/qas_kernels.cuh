@@ -319,13 +319,23 @@ static __global__ void k_dv(View v)
 #define QAS_LR_MINB 7
 #endif
 
+// NC: through the non-coherent path, which asks for data that nobody writes during the kernel's life: only in
+// kernels launched without overlap.  One launched with it (pdl_begin) starts while its predecessor still writes
+// the fields and takes plain loads.  Plain / non-coherent with the launch each needs, us a step: KH 160^3 8086 /
+// 8029, OT 1024^2 1173 / 1184, KH 360^2 HLLD as single launches 210 / 225: the sweeps overlap.  Not so the Athena-type
+// form, whose spills grow with plain loads (KH 400^2 352 / 341), nor the ensemble's kernels (24 grids of 64..512
+// 2030 / 2007).
+template <bool NC>
+__device__ __forceinline__ double ld(const double *p)
+{
+  if constexpr (NC) return __ldg(p);
+  return *p;
+}
+
 // stencil accessor of k_lr: field f of (ro, vn, vb, vc, cb, cc, pr) along axis A at point m
 // (0..4) of cell c; the field pointers are read from the kernel's View parameter at each use,
-// so no pointer stays live in registers.  Plain loads, here and in the sweeps: a launch that overlaps its
-// predecessor (pdl_begin) starts while that one still writes these fields, and the non-coherent path (__ldg)
-// asks for data that nobody writes during the kernel's life.  A step with plain / non-coherent loads, us: KH
-// 160^3 8075 / 8015, KH 117x75x93 1918 / 1907, OT 1024^2 1172 / 1174, KH 64^3 at the 2nd order 559 / 575.
-template <int A>
+// so no pointer stays live in registers
+template <int A, bool NC>
 struct LrStencil {
   const View &v;
   unsigned c, s;  // byte offset of the cell, byte stride of the axis
@@ -346,7 +356,7 @@ struct LrStencil {
       default: return v.pr;
     }
   }
-  __device__ __forceinline__ double operator()(int f, int m) const { return *at(field(f), c + (m - 2) * s); }
+  __device__ __forceinline__ double operator()(int f, int m) const { return ld<NC>(at(field(f), c + (m - 2) * s)); }
 };
 
 // face_states of cell c along A by the reference's divisions, out of line: what the kernels call for
@@ -355,7 +365,7 @@ struct LrStencil {
 template <int ODR, int A>
 __device__ __noinline__ void states_again(const View &v, long long c, double *l, double *r, long long ls)
 {
-  const LrStencil<A> st{v, c, v.g.s[A]};
+  const LrStencil<A, false> st{v, c, v.g.s[A]};
   double vl[7], vr[7];
   face_states_of<ODR>(st, (A == 0 ? v.cx : (A == 1 ? v.cy : v.cz))[c], v.gam, vl, vr);
   for (int m = 0; m < 7; m++) {
@@ -429,7 +439,7 @@ __device__ __forceinline__ void lr_cell(const View &v, long long c, long long s,
   }
 }
 
-template <int ODR, int A, int PR = -1>
+template <int ODR, int A, int PR = -1, bool NC = false>
 __device__ __forceinline__ void lr_body(const View &v, int i, int j, int k)
 {
   const Geo &g = v.g;
@@ -439,16 +449,19 @@ __device__ __forceinline__ void lr_body(const View &v, int i, int j, int k)
   const long long c = cidx(g, i, j, k);
   const long long s = g.s[A];
   const double *cn = A == 0 ? v.cx : (A == 1 ? v.cy : v.cz);
-  const LrStencil<A> st{v, c, s};
+  const LrStencil<A, NC> st{v, c, s};
   lr_cell<ODR, A, PR>(v, c, s, st, cn[c]);
 }
+// the Athena-type form: no overlap (ld), 6 blocks (80 registers), at which the 2nd order's spills nearly go: KH 400^2 /
+// 64^3 HLLD at 7 / 6 blocks, us a step, 254 / 237 and 824 / 784
+#define QAS_LR_ATHENA(PR) ((PR) == 2)
 template <int ODR, int A, int PR = 0>
-__global__ void __launch_bounds__(128, QAS_LR_MINB) k_lr(const __grid_constant__ View v)
+__global__ void __launch_bounds__(128, QAS_LR_ATHENA(PR) ? 6 : QAS_LR_MINB) k_lr(const __grid_constant__ View v)
 {
   pdl_begin();
   if (v.ctl->done) return;
   QAS_CELL_INDEX();
-  lr_body<ODR, A, PR>(v, i, j, k);
+  lr_body<ODR, A, PR, QAS_LR_ATHENA(PR)>(v, i, j, k);
 }
 
 // ---------------------------------------------------------------------------
@@ -638,27 +651,27 @@ struct StatesToSlots {
 
 // states of cell c: right face into the slots l[m * SLP], left face into r[m * SLP] (m < SLOTS).
 // PR: 0 the characteristic or primitive form by v.recon, -1 any of the three
-template <int ODR, int A, int PR>
+template <int ODR, int A, int PR, bool NC>
 __device__ __forceinline__ void cell_states(const View &v, long long c, double *l, double *r)
 {
   const Geo &g = v.g;
   const long long s = g.s[A];
   const double *cn = A == 0 ? v.cx : (A == 1 ? v.cy : v.cz);
-  const LrStencil<A> st{v, c, s};
+  const LrStencil<A, NC> st{v, c, s};
   const StatesToSlots<ODR, A> store{v, c, l, r};
   if ((PR <= 0 && v.recon == 1) || (PR < 0 && v.recon == 2)) {
     double vl[7], vr[7];
     if (PR < 0 && v.recon == 2)
-      face_states_athena<ODR>(st, *at(cn, st.c), v.gam, vl, vr);
+      face_states_athena<ODR>(st, ld<NC>(at(cn, st.c)), v.gam, vl, vr);
     else
       face_states_prim<ODR>(st, vl, vr);
 #pragma unroll
     for (int m = 0; m < 7; m++) store(m, vl[m], vr[m]);
   } else {
-    face_states_emit<ODR>(st, *at(cn, st.c), v.gam, store);
+    face_states_emit<ODR>(st, ld<NC>(at(cn, st.c)), v.gam, store);
   }
   if (g.dim >= 2) {
-    const double bfl = *at(v.u[4 + A], st.c + st.s), bfr = *at(v.u[4 + A], st.c);
+    const double bfl = ld<NC>(at(v.u[4 + A], st.c + st.s)), bfr = ld<NC>(at(v.u[4 + A], st.c));
 #pragma unroll
     for (int t = 0; t < 2; t++) {
       if (g.dim == 2 && ((A == 0 && t == 1) || (A == 1 && t == 0))) continue;
@@ -678,24 +691,24 @@ __device__ __forceinline__ void cell_states(const View &v, long long c, double *
 
 // flux at face f from the left cell's right-face state, slots l[m * SLP], and this cell's left-face
 // state, slots r[m * SLP]
-template <int RMN, int A>
+template <int RMN, int A, bool NC>
 __device__ __forceinline__ void face_flux(const View &v, long long f, const double *l, const double *r)
 {
   const Geo &g = v.g;
   const long long s = g.s[A];
   constexpr int B = (A + 1) % 3, C = (A + 2) % 3;
   const unsigned o = (unsigned)(8 * f), so = (unsigned)(8 * s);
-  const double bn = *at(v.u[4 + A], o);  // the reference's 0.5*(bn + bn)
+  const double bn = ld<NC>(at(v.u[4 + A], o));  // the reference's 0.5*(bn + bn)
   double dv0 = 0.0, dv1 = 0.0;
   if (RMN >= 2) {
     const double *vn = A == 0 ? v.vx : (A == 1 ? v.vy : v.vz);
-    dv0 = *at(vn, o) - *at(vn, o - so);
+    dv0 = ld<NC>(at(vn, o)) - ld<NC>(at(vn, o - so));
     if (g.dim == 2) {
       const double *dt = v.dv[A == 0 ? 1 : 0];
-      dv1 = qmin(*at(dt, o - so), *at(dt, o));
+      dv1 = qmin(ld<NC>(at(dt, o - so)), ld<NC>(at(dt, o)));
     } else if (g.dim == 3) {
       const double *d1 = v.dv[B], *d2 = v.dv[C];
-      dv1 = qmin(qmin(*at(d1, o - so), *at(d1, o)), qmin(*at(d2, o - so), *at(d2, o)));
+      dv1 = qmin(qmin(ld<NC>(at(d1, o - so)), ld<NC>(at(d1, o))), qmin(ld<NC>(at(d2, o - so)), ld<NC>(at(d2, o))));
     }
   }
   double L[7], R[7];
@@ -710,14 +723,14 @@ __device__ __forceinline__ void face_flux(const View &v, long long f, const doub
 // one lane of an x-sweep warp: the face states of cell (i, j, k) (a valid cell even for a lane
 // past the end, have_cell false, so that the warp stays converged) and the flux at the cell's
 // left face when the previous lane holds the cell to its left (i >= 3)
-template <int ODR, int RMN, int PR>
+template <int ODR, int RMN, int PR, bool NC>
 __device__ __forceinline__ void sweep_x_cell(const View &v, int i, int j, int k, int lane, bool have_cell, double *sm)
 {
   const long long c = cidx(v.g, i, j, k);
   double *l = sm + threadIdx.x, *r = l + SWB;
-  cell_states<ODR, 0, PR>(v, c, l, r);
+  cell_states<ODR, 0, PR, NC>(v, c, l, r);
   __syncwarp();
-  if (lane >= 1 && have_cell && i >= 3) face_flux<RMN, 0>(v, c, l - 1, r);
+  if (lane >= 1 && have_cell && i >= 3) face_flux<RMN, 0, NC>(v, c, l - 1, r);
 }
 
 __device__ __forceinline__ void prefetch_l1(const double *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
@@ -727,7 +740,7 @@ __device__ __forceinline__ void prefetch_l1(const double *p) { asm volatile("pre
 // before p0 on.  The block's warps take consecutive cells, so that they share their stencils' lines
 // in L1; warp w's cell is handed to warp w + 1 through row w + 1 of the slots, the last warp's
 // to the next round through row 0.
-template <int ODR, int RMN, int A, int PR>
+template <int ODR, int RMN, int A, int PR, bool NC>
 __device__ __forceinline__ void sweep_columns(const View &v, int i, int o, bool have, int p0, int p1, double *sm)
 {
   constexpr int NW = SWB / 32;
@@ -749,15 +762,15 @@ __device__ __forceinline__ void sweep_columns(const View &v, int i, int o, bool 
       prefetch_l1(v.dv[C] + c);
       prefetch_l1(v.u[4 + A] + c);
     }
-    if (cell) cell_states<ODR, A, PR>(v, c, l + 32, r);
+    if (cell) cell_states<ODR, A, PR, NC>(v, c, l + 32, r);
     if (have && p + NW + w < p1) {  // the plane that this warp's next stencil adds
       const long long q = c + (NW + 2) * s;
-      const LrStencil<A> st{v, c, s};
+      const LrStencil<A, NC> st{v, c, s};
 #pragma unroll
       for (int f = 0; f < 7; f++) prefetch_l1(at(st.field(f), (unsigned)(8 * q)));
     }
     __syncthreads();
-    if (cell && p + w >= p0) face_flux<RMN, A>(v, c, l, r);
+    if (cell && p + w >= p0) face_flux<RMN, A, NC>(v, c, l, r);
     __syncthreads();
     c += NW * s;
   }
@@ -773,7 +786,7 @@ struct SweepPlan {
 
 // block `blk` of a sweep over the axes AX (bit a).  The y / z blocks march over `seg` faces of 32 columns;
 // an x warp takes 31 faces of the flattened cells of all rows.
-template <int ODR, int RMN, int PR, int AX>
+template <int ODR, int RMN, int PR, int AX, bool NC>
 __device__ __forceinline__ void sweep_block(const View &v, const SweepPlan &pl, unsigned blk, double *sm)
 {
   const Geo &g = v.g;
@@ -790,10 +803,10 @@ __device__ __forceinline__ void sweep_block(const View &v, const SweepPlan &pl, 
     const int p0 = 3 + (int)s * pl.seg[q], p1 = min(p0 + pl.seg[q], g.n[1 + q] - 2);
     const int i = (int)(col % g.nx), o = (int)(col / g.nx);
     if constexpr ((AX & 4) != 0) {
-      if (z) sweep_columns<ODR, RMN, 2, PR>(v, i, o, have, p0, p1, sm);
+      if (z) sweep_columns<ODR, RMN, 2, PR, NC>(v, i, o, have, p0, p1, sm);
     }
     if constexpr ((AX & 2) != 0) {
-      if (!z) sweep_columns<ODR, RMN, 1, PR>(v, i, o, have, p0, p1, sm);
+      if (!z) sweep_columns<ODR, RMN, 1, PR, NC>(v, i, o, have, p0, p1, sm);
     }
     return;
   }
@@ -807,7 +820,7 @@ __device__ __forceinline__ void sweep_block(const View &v, const SweepPlan &pl, 
   const bool have_cell = t < total;
   if (!have_cell) t = total - 1;  // a valid cell, computed and discarded (keeps the warp converged)
   const unsigned row = t / ncell, k = row / g.ny;
-  sweep_x_cell<ODR, RMN, PR>(v, 2 + (t - row * ncell), row - k * g.ny, k, lane, have_cell, sm);
+  sweep_x_cell<ODR, RMN, PR, NC>(v, 2 + (t - row * ncell), row - k * g.ny, k, lane, have_cell, sm);
 }
 
 // the sweep kernel (qas_sweep.cu) of an order (2 or 4), solver, reconstruction form (any: all three, else

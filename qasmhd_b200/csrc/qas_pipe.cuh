@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(SWB, QAS_SWEEP_MINB_OF(RMN)) kw_sweep_x(const 
   const int i = 2 + (t - row * ncell);
   const int j = g.dim == 3 ? (int)(row - plane * per_plane) : rows2_plane(r, (int)row);
   const int k = g.dim == 3 ? rows2_plane(r, (int)plane) : 0;
-  sweep_x_cell<ODR, RMN, PR>(v, i, j, k, lane, have_cell, sm);
+  sweep_x_cell<ODR, RMN, PR, false>(v, i, j, k, lane, have_cell, sm);
 }
 
 // y sweep of a 3D window (an in-plane axis): columns (i, k) with k on planes r, every y face
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(SWB, QAS_SWEEP_MINB_OF(RMN)) kw_sweep_y3(const
   const bool have = col < cols;
   if (!have) col = cols - 1;
   const int p0 = 3 + blockIdx.y * seg;
-  sweep_columns<ODR, RMN, 1, PR>(v, (int)(col % g.nx), rows2_plane(r, (int)(col / g.nx)), have, p0,
+  sweep_columns<ODR, RMN, 1, PR, false>(v, (int)(col % g.nx), rows2_plane(r, (int)(col / g.nx)), have, p0,
                              min(p0 + seg, g.ny - 2), sm);
 }
 
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(SWB, QAS_SWEEP_MINB_OF(RMN)) kw_sweep_last(con
   const Rows &x = q < ca ? a : b;
   const int p0 = x.lo + (q < ca ? q : q - ca) * seg;
   if (p0 >= x.hi) return;  // the whole block
-  sweep_columns<ODR, RMN, A, PR>(v, (int)(col % g.nx), (int)(col / g.nx), have, p0, min(p0 + seg, x.hi), sm);
+  sweep_columns<ODR, RMN, A, PR, false>(v, (int)(col % g.nx), (int)(col / g.nx), have, p0, min(p0 + seg, x.hi), sm);
 }
 
 template <int ODR>

@@ -14,7 +14,7 @@ __global__ void __launch_bounds__(SWB, QAS_SWEEP_MINB_OF(RMN)) k_sweep(const __g
   pdl_begin();
   if (v.ctl->done) return;
   __shared__ double sm[SLOTS * SLP];
-  sweep_block<ODR, RMN, PR, AX>(v, pl, blockIdx.x, sm);
+  sweep_block<ODR, RMN, PR, AX, (PR < 0)>(v, pl, blockIdx.x, sm);
 }
 
 template <int ODR, int PR, int AX>

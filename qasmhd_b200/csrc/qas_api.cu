@@ -11,6 +11,7 @@
 #include <cstdio>
 #include <cstring>
 #include <exception>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -92,7 +93,11 @@ static qas_status pipe_set_lanes(qas_ctx *c, int value);
 
 // Streams of a graph capture on which independent launches (the face sweeps of the axes) become parallel
 // branches: fork() after the launch they depend on, stream(i) for the branches beside the main one, join()
-// before the launch that needs them all.  Temporary: the captured graph keeps no stream or event.
+// before the launch that needs them all.  Temporary: the captured graph keeps no stream or event.  The streams
+// and events cost 0.35 ms of a capture, a graph with branches 0.1-0.4 ms more at its first launch and its end, so a
+// capture takes them only where more steps follow (CAPTURE_STEPS).  One stream whose capture's end is set back
+// for each branch needs no others, but its graph's first launch and end then cost as much (RT 128x512, create to
+// close with 4 steps, 0.2 ms more).
 struct Branches {
   static constexpr int N = 3;
   cudaStream_t st[N] = {};
@@ -132,6 +137,13 @@ struct Branches {
   }
 };
 
+// steps from which a call's capture has branches at once.  A call of fewer, the first with its options, captures
+// the launches one after the other, the next call (of an ensemble: one that brings the steps to this number) with
+// branches: a program that makes a context, runs a few steps and closes it pays for no more than it uses.  The first
+// call of 4 steps, with branches / without, us: RT 128x512 1380 / 1050, OT 400x300 1377 / 1064, KH 48^3 2485 / 1891,
+// OT 1024^2 5276 / 5016, 4 grids of 64..128 2123 / 1267.
+constexpr int CAPTURE_STEPS = 32;
+
 struct qas_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -158,6 +170,7 @@ struct qas_ctx {
   double graph_cfl = 0.0, graph_nu0 = -1.0, graph_eta0 = -1.0, graph_dtrec = 0.0;
   int graph_nout = 0;
   unsigned graph_form = 0;  // stage_form() of its steps
+  bool graph_branched = false;
   long long graph_kernels = 0;
   long long launches = 0;
   bool capturing = false;
@@ -744,6 +757,12 @@ long long stage_dv(qas_ctx *c)
   QL(c, KID_DV, launch(c, k_dv, cells_grid(c->geo, c->tile[KID_DV]), c->tile[KID_DV], c->view));
   return 1;
 }
+// whether a captured step can run its face sweeps side by side
+bool step_branches(const qas_ctx *c)
+{
+  const unsigned axes = c->fused & ((1u << c->geo.dim) - 1u);
+  return c->scheme.odr == 4 && c->geo.dim >= 2 && (axes & 1u) && (c->geo.dim == 2 || axes == 7u);
+}
 template <int ODR>
 long long stage_rest(qas_ctx *c, double c0, double c1)
 {
@@ -762,12 +781,11 @@ long long stage_rest(qas_ctx *c, double c0, double c1)
     }
     nk += 2;
   };
-  // at most one axis writes the face-state arrays: its launches and the sweeps of the others touch nothing in
-  // common and become branches of the captured step, which fills each launch's last wave and, on small grids,
+  // step_branches: at most one axis writes the face-state arrays, its launches and the sweeps of the others touch
+  // nothing in common and become branches of the captured step, which fills each launch's last wave and, on small grids,
   // idle SMs.  One after the other / side by side, us a step: RT 128x512 188 / 183, OT 512x400 336 / 326, OT
   // 1024^2 1173 / 1159, KH 117x75x93 1973 / 1879, KH 160^3 7952 / 7907
-  const bool branches = ODR == 4 && c->branch && g.dim >= 2 && (axes & 1u) && (g.dim == 2 || axes == 7u);
-  if (branches) {
+  if (c->branch) {
     cudaStream_t outer = c->stream;
     c->branch->fork(outer, g.dim - 1);
     nk += launch_sweep(c, axes & 1u);
@@ -1568,28 +1586,31 @@ qas_status qas_run(qas_ctx *c, const qas_run_opts *opts, qas_run_info *info)
   }
   const bool want_graph = o.use_graph != 0 && !hall_active(c);  // the Hall sub-cycle count is read back
   if (want_graph && launched + 2 <= limit) {
-    const bool stale = !c->graph || c->graph_flg != o.flg || c->graph_rule != o.stop_rule || c->graph_cfl != o.cfl ||
-                       c->graph_nu0 != o.nu0 || c->graph_eta0 != o.eta0 || c->graph_dtrec != o.dtrec ||
-                       c->graph_nout != o.nout || c->graph_form != stage_form(c);
-    if (stale) {
+    const bool same = c->graph && c->graph_flg == o.flg && c->graph_rule == o.stop_rule && c->graph_cfl == o.cfl &&
+                      c->graph_nu0 == o.nu0 && c->graph_eta0 == o.eta0 && c->graph_dtrec == o.dtrec &&
+                      c->graph_nout == o.nout && c->graph_form == stage_form(c);
+    const bool branched = step_branches(c) && (same || limit - launched >= CAPTURE_STEPS);
+    if (!same || (branched && !c->graph_branched)) {
       if (c->graph) {
         cudaGraphExecDestroy(c->graph);
         c->graph = nullptr;
+      }
+      std::unique_ptr<Branches> side(branched ? new Branches() : nullptr);
+      if (side && side->err != cudaSuccess) {  // no stream to be had: one after the other
+        cudaGetLastError();
+        side.reset();
       }
       cudaGraph_t gph;
       QAS_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
       const bool diss = o.nu0 > 0.0 || o.eta0 > 0.0 || diss_arrays(c);  // a loop node takes plain edges
       c->plain_edges = c->geo.nd < (1 << 17) || diss;
       c->capture_err = cudaSuccess;
-      Branches side;
-      const bool fork = side.err == cudaSuccess;
-      if (side.err != cudaSuccess) cudaGetLastError();
-      c->branch = fork ? &side : nullptr;
+      c->branch = side.get();
       c->capturing = true;
       long long nk = launch_exec_step(c, o, 1, fill) + launch_exec_step(c, o, 2, fill);
       c->capturing = false;
       c->branch = nullptr;
-      if (fork && c->capture_err == cudaSuccess) c->capture_err = side.err;
+      if (side && c->capture_err == cudaSuccess) c->capture_err = side->err;
       cudaError_t e = cudaStreamEndCapture(c->stream, &gph);
       if (c->capture_err != cudaSuccess) {
         if (e == cudaSuccess && gph) cudaGraphDestroy(gph);
@@ -1608,6 +1629,7 @@ qas_status qas_run(qas_ctx *c, const qas_run_opts *opts, qas_run_info *info)
       c->graph_dtrec = o.dtrec;
       c->graph_nout = o.nout;
       c->graph_form = stage_form(c);
+      c->graph_branched = branched;
     }
   }
   const int chunk = 32;  // steps between host checks of the stop flag

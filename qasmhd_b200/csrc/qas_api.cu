@@ -1087,10 +1087,15 @@ bool ghosts_kept(const qas_ctx *c) { return !c->view.phi && !hall_active(c); }
 
 // 1D steps in one kernel a stage (qas_stage1d.cuh): the orders it is built for, at least two stages (a
 // block's neighbours read its cells while it writes), no Hall form, no form asked for or timed apart.
-// Brio-Wu 1024: 62.7 us a step in 17 launches, 22.6 us in 3.
+// Brio-Wu 1024: 62.7 us a step in 17 launches, 22.6 us in 3.  On large grids launches no longer count, but the eight
+// cells in 64 that a block computes for its neighbours and the low occupancy do; one kernel / separate ones, us a
+// step: 4th order, 20 k cells HLLD 27 / 62, 262 k Roe 179 / 182, HLLD 159 / 167, LHLLD 167 / 175, MLAU 205 / 190, 400 k
+// 283 / 274, 255 / 249, 261 / 260, 320 / 282, 10^6 HLLD 663 / 546; 2nd order, Roe 262 k 136 / 140, 400 k 225 / 212, HLLD
+// 600 k 250 / 258, 2 M 795 / 790, LHLLD 2 M 834 / 845, 8 M 3231 / 3150, MLAU 8 M 3101 / 3553.
 bool one_kernel_stages(const qas_ctx *c)
 {
-  return c->geo.dim == 1 && (c->scheme.odr == 4 || c->scheme.odr == 2) && c->scheme.rk >= 2 &&
+  const long long most = c->scheme.odr == 4 || c->scheme.rmn == 0 ? 1ll << 18 : c->scheme.rmn == 3 ? LLONG_MAX : 1ll << 21;
+  return c->geo.dim == 1 && c->geo.nd <= most && (c->scheme.odr == 4 || c->scheme.odr == 2) && c->scheme.rk >= 2 &&
          c->scheme.char_mode != 2 && !c->hall && !c->fused_set && !c->prof;
 }
 // everything that decides which kernels a step consists of and an option can change between two runs: a

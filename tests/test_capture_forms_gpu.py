@@ -44,3 +44,15 @@ def test_calls_of_an_ensemble(restatement, calls, odr):
         for q, p in enumerate(probs):
             want = restatement.run(p, sum(calls), mode=R.MODE_RUN)["state"]
             assert_bitwise(b.download(q, p.state.shape), want, f"{p.name} {calls}")
+
+
+@pytest.mark.parametrize("n", [(1 << 18) - 8, (1 << 18) - 7])
+@pytest.mark.parametrize("rmn,odr", [(1, 4), (0, 2), (3, 2)])
+def test_1d_stage_form_by_size(restatement, n, rmn, odr):
+    """The padded sizes on either side of the line between one kernel a stage and separate ones."""
+    p = P.smooth_wave(1, n, amp=0.1, rmn=rmn, odr=odr)
+    want = restatement.run(p, 3, mode=R.MODE_RUN)["state"]
+    with L.Context.from_problem(p) as ctx:
+        ctx.upload(p.state)
+        ctx.run(max_steps=3, flg=p.flg, cfl=p.cfl)
+        assert_bitwise(ctx.download(p.state.shape), want, f"{n} {rmn} {odr}")

@@ -664,13 +664,15 @@ void sweep_prepare(qas_ctx *c)
 // the axes whose face states stay on chip by default (bit a).  3D: all.  2D: x, and y for the HLLD
 // solvers and on small grids, where a launch counts more than the march (OT / KH 1024^2, two kernels
 // against one, us: x HLLD 139 / 121, LHLLD 149 / 134, MLAU 152 / 139, Roe 162 / 162; y HLLD 138 / 136,
-// LHLLD 152 / 147, MLAU 147 / 157, Roe 161 / 178).  1D: none.
+// LHLLD 152 / 147, MLAU 147 / 157, Roe 161 / 178).  The line for y, KH, two kernels / fused, us a step of Roe and of
+// MLAU: 160^2 116 / 113, 125 / 122; 256^2 155 / 156, 160 / 161; 300^2 184 / 176, 187 / 186; 400^2 252 / 255, 249 / 250;
+// 450^2 305 / 306, 299 / 314; 100x2000 321 / 328, 315 / 333; 600^2 493 / 508, 472 / 488.  1D: none.
 unsigned fused_axes(const qas_ctx *c)
 {
   if (!sweep_built(c) || c->geo.dim == 1) return 0u;
   if (c->geo.dim == 3 || c->scheme.odr == 2) return 7u;
   const bool hlld = c->scheme.rmn == 1 || c->scheme.rmn == 2;
-  return hlld || c->geo.nd <= (1ll << 18) ? 3u : 1u;
+  return hlld || c->geo.nd <= (1ll << 17) ? 3u : 1u;
 }
 
 // the blocks of a sweep over the axes

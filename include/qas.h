@@ -289,6 +289,9 @@ qas_status qas_set_gravity(qas_ctx *ctx, const double *phi_g);
  * reports QAS_ERR_TIMEOUT (the state is then not a valid step).  value < 0 restores the defaults.
  * QAS_ERR_UNSUPPORTED where the staged form is not available. */
 #define QAS_OPT_TEST_TMA_STALL 5
+/* Failure-path hook: value != 0 makes the loop node of a captured dissipative step fail as on a driver without
+ * conditional nodes, so that qas_run captures the guarded sub-cycles instead; 0 restores the default. */
+#define QAS_OPT_TEST_NO_LOOP 6
 qas_status qas_set_option(qas_ctx *ctx, int option, int value);
 
 /* Thread-block tile (tx*ty*tz <= 128 threads, tx a multiple of 32) of one cell kernel

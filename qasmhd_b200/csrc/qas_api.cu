@@ -178,6 +178,8 @@ struct qas_ctx {
   bool plain_next = false;     // the launches of a branch and of a join: plain edges
   bool plain_edges = false;  // the graph being captured takes plain edges (launch)
   cudaError_t capture_err = cudaSuccess;  // of a call inside the capture
+  bool sub_loop = true;       // a captured step's sub-cycles are a loop node (false: one could not be made)
+  bool test_no_loop = false;  // QAS_OPT_TEST_NO_LOOP
   qas_status latched = QAS_OK;
   // thread-block tile (x,y,z extents, 128 threads) of every cell kernel, by kernel id
   dim3 tile[32];
@@ -977,7 +979,8 @@ cudaError_t capture_subcycles(qas_ctx *c, cudaGraph_t graph, cudaGraphConditiona
 
 // setdc + sub-cycled dsptv after ideal (dmhd2d_class.cpp:19-26, dmhd3d_class.cpp:20-28): issued eagerly,
 // NSUB_CAP sub-cycles that the device guards; in a graph, the loop above (KH 515x301, one sub-cycle of the eight:
-// 12 kernels instead of 136).  fill: the ghosts may not be filled yet
+// 12 kernels instead of 136), or the guarded ones where the loop cannot be made (c->sub_loop).  fill: the ghosts may
+// not be filled yet
 long long launch_dissipate(qas_ctx *c, double nu0, double eta0, bool fill)
 {
   // setdc's maximum of max(2 nu, eta) over every cell: the installed profiles, else uniform
@@ -987,12 +990,14 @@ long long launch_dissipate(qas_ctx *c, double nu0, double eta0, bool fill)
   const double idz = c->grid.dim == 3 ? 1.0 / c->grid.dz : 0.0;
   cudaGraphConditionalHandle loop = 0;
   cudaGraph_t graph = nullptr;
-  if (c->capturing) {
+  const bool in_graph = c->capturing && c->sub_loop;
+  if (in_graph) {
     cudaStreamCaptureStatus st;
     const cudaGraphNode_t *deps = nullptr;
     const cudaGraphEdgeData *edges = nullptr;
     size_t nd = 0;
-    cudaError_t e = cudaStreamGetCaptureInfo_v3(c->stream, &st, nullptr, &graph, &deps, &edges, &nd);
+    cudaError_t e = c->test_no_loop ? cudaErrorNotSupported : cudaSuccess;
+    if (e == cudaSuccess) e = cudaStreamGetCaptureInfo_v3(c->stream, &st, nullptr, &graph, &deps, &edges, &nd);
     if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&loop, graph, 0, cudaGraphCondAssignDefault);
     if (e != cudaSuccess) {
       c->capture_err = e;
@@ -1002,7 +1007,7 @@ long long launch_dissipate(qas_ctx *c, double nu0, double eta0, bool fill)
   QL(c, KID_DSUB, launch(c, k_dsub_setup, 1, 1, c->view, c->d_dctl, dcmax, c->dr, 1.0 / c->grid.dx,
                          1.0 / c->grid.dy, NSUB_CAP, idz, loop));
   long long nk = 1;
-  if (c->capturing) {
+  if (in_graph) {
     const cudaError_t e = capture_subcycles(c, graph, loop, nu0, eta0, nk);
     if (e != cudaSuccess) c->capture_err = e;
     return nk;
@@ -1536,6 +1541,37 @@ qas_status qas_run_reset(qas_ctx *c)
   QAS_API_CATCH
 }
 
+static bool dissipative(const qas_ctx *c, const qas_run_opts &o) { return o.nu0 > 0.0 || o.eta0 > 0.0 || diss_arrays(c); }
+
+// c->graph: two exec_ steps, odd then even n, their face sweeps as branches or one after the other
+static cudaError_t capture_steps(qas_ctx *c, const qas_run_opts &o, bool fill, bool branched, long long &nk)
+{
+  std::unique_ptr<Branches> side(branched ? new Branches() : nullptr);
+  if (side && side->err != cudaSuccess) {  // no stream to be had: one after the other
+    cudaGetLastError();
+    side.reset();
+  }
+  cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
+  if (e != cudaSuccess) return e;
+  c->plain_edges = c->geo.nd < (1 << 17) || dissipative(c, o);  // a loop node takes plain edges
+  c->capture_err = cudaSuccess;
+  c->branch = side.get();
+  c->capturing = true;
+  nk = launch_exec_step(c, o, 1, fill) + launch_exec_step(c, o, 2, fill);
+  c->capturing = false;
+  c->branch = nullptr;
+  if (side && c->capture_err == cudaSuccess) c->capture_err = side->err;
+  cudaGraph_t gph = nullptr;
+  e = cudaStreamEndCapture(c->stream, &gph);
+  if (c->capture_err != cudaSuccess) e = c->capture_err;
+  if (e == cudaSuccess) {
+    e = cudaGraphInstantiate(&c->graph, gph, 0);
+    if (e != cudaSuccess) c->graph = nullptr;
+  }
+  if (gph) cudaGraphDestroy(gph);
+  return e;
+}
+
 static qas_status end_run(qas_ctx *c, int n0, qas_run_info *info)
 {
   const qas_status s = read_ctl(c);
@@ -1602,31 +1638,14 @@ qas_status qas_run(qas_ctx *c, const qas_run_opts *opts, qas_run_info *info)
         cudaGraphExecDestroy(c->graph);
         c->graph = nullptr;
       }
-      std::unique_ptr<Branches> side(branched ? new Branches() : nullptr);
-      if (side && side->err != cudaSuccess) {  // no stream to be had: one after the other
+      long long nk = 0;
+      cudaError_t e = capture_steps(c, o, fill, branched, nk);
+      if (e != cudaSuccess && c->sub_loop && dissipative(c, o)) {  // no loop node to be had
         cudaGetLastError();
-        side.reset();
-      }
-      cudaGraph_t gph;
-      QAS_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-      const bool diss = o.nu0 > 0.0 || o.eta0 > 0.0 || diss_arrays(c);  // a loop node takes plain edges
-      c->plain_edges = c->geo.nd < (1 << 17) || diss;
-      c->capture_err = cudaSuccess;
-      c->branch = side.get();
-      c->capturing = true;
-      long long nk = launch_exec_step(c, o, 1, fill) + launch_exec_step(c, o, 2, fill);
-      c->capturing = false;
-      c->branch = nullptr;
-      if (side && c->capture_err == cudaSuccess) c->capture_err = side->err;
-      cudaError_t e = cudaStreamEndCapture(c->stream, &gph);
-      if (c->capture_err != cudaSuccess) {
-        if (e == cudaSuccess && gph) cudaGraphDestroy(gph);
-        return cuda_fail(c->capture_err, "graph capture");
+        c->sub_loop = false;
+        e = capture_steps(c, o, fill, branched, nk);
       }
       if (e != cudaSuccess) return cuda_fail(e, "graph capture");
-      e = cudaGraphInstantiate(&c->graph, gph, 0);
-      cudaGraphDestroy(gph);
-      if (e != cudaSuccess) return cuda_fail(e, "graph instantiate");
       c->graph_kernels = nk;
       c->graph_flg = o.flg;
       c->graph_rule = o.stop_rule;
@@ -1941,6 +1960,15 @@ qas_status qas_set_gravity(qas_ctx *c, const double *phi_g)
   QAS_API_CATCH
 }
 
+static void drop_graph(qas_ctx *c)
+{
+  if (c->graph) {
+    cudaStreamSynchronize(c->stream);
+    cudaGraphExecDestroy(c->graph);
+    c->graph = nullptr;
+  }
+}
+
 qas_status qas_set_option(qas_ctx *c, int option, int value)
 {
   QAS_API_TRY
@@ -1973,6 +2001,12 @@ qas_status qas_set_option(qas_ctx *c, int option, int value)
     }
     return QAS_OK;
   }
+  if (option == QAS_OPT_TEST_NO_LOOP) {
+    drop_graph(c);
+    c->test_no_loop = value != 0;
+    c->sub_loop = true;
+    return QAS_OK;
+  }
   if (option == QAS_OPT_PIPE_ITEMS) return pipe_set_items(c, value);
   if (option == QAS_OPT_PIPE_LANES) return pipe_set_lanes(c, value);
   return QAS_ERR_INVALID;
@@ -1987,15 +2021,6 @@ static int tile_kid(const char *k)
   for (int q = 0; q < 6; q++)
     if (!strcmp(k, KID_NAMES[kids[q]])) return kids[q];
   return -2;
-}
-
-static void drop_graph(qas_ctx *c)
-{
-  if (c->graph) {
-    cudaStreamSynchronize(c->stream);
-    cudaGraphExecDestroy(c->graph);
-    c->graph = nullptr;
-  }
 }
 
 qas_status qas_set_tile(qas_ctx *c, const char *kernel, int tx, int ty, int tz)

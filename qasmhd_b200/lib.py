@@ -49,6 +49,7 @@ QAS_OPT_LR_STAGING = 2
 QAS_OPT_PIPE_ITEMS = 3
 QAS_OPT_PIPE_LANES = 4
 QAS_OPT_TEST_TMA_STALL = 5
+QAS_OPT_TEST_NO_LOOP = 6
 
 
 class QasError(RuntimeError):

@@ -56,3 +56,21 @@ def test_1d_stage_form_by_size(restatement, n, rmn, odr):
         ctx.upload(p.state)
         ctx.run(max_steps=3, flg=p.flg, cfl=p.cfl)
         assert_bitwise(ctx.download(p.state.shape), want, f"{n} {rmn} {odr}")
+
+
+@pytest.mark.parametrize("case", ["kh2d_roe_eta", "kh3d_hlld_eta"])
+def test_captured_subcycles_without_a_loop_node(restatement, case):
+    """Where the loop node cannot be made the captured step holds the guarded sub-cycles."""
+    make, eta = CASES[case]
+    p = make()
+    p.eta0 = eta
+    with L.Context.from_problem(p) as ctx:
+        ctx.upload(p.state)
+        n = 0
+        for steps, no_loop in ((4, 1), (4, None), (3, 0)):  # the second call's capture has branches
+            if no_loop is not None:
+                ctx.set_option(L.QAS_OPT_TEST_NO_LOOP, no_loop)
+            ctx.run(max_steps=steps, flg=p.flg, cfl=p.cfl, eta0=eta)
+            n += steps
+            want = restatement.run(p, n, mode=R.MODE_DRUN)["state"]
+            assert_bitwise(ctx.download(p.state.shape), want, f"{case} {n} steps")

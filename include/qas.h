@@ -230,8 +230,10 @@ qas_status qas_bc_map(const qas_grid *grid, const qas_bc *bc, int group, int fie
 /* Diagnostics: per-kernel device time measured live with CUDA events on the context's
  * stream.  Runs `nsteps` exec_ steps (the same work as qas_run, launched eagerly) with an
  * event pair around every kernel launch and returns, per kernel, the number of launches and
- * the summed durations (in 2D with the face sweeps in their two-kernel form unless
- * QAS_OPT_FUSED_SWEEP was set, so that the reconstruction and the flux are timed apart).  *count receives the number of entries written (<= max_entries). */
+ * the summed durations.  In 2D the face sweeps are timed in their two-kernel form, the
+ * reconstruction and the flux apart, unless QAS_OPT_FUSED_SWEEP or QAS_OPT_PROFILE_AS_RUN was
+ * set; elsewhere the kernels are those of qas_run.  *count receives the number of entries
+ * written (<= max_entries). */
 typedef struct {
   char name[32];
   long long launches;
@@ -267,10 +269,13 @@ qas_status qas_set_gravity(qas_ctx *ctx, const double *phi_g);
 
 /* Tuning options (defaults are the measured best on B200).
  *   QAS_OPT_FUSED_SWEEP: 0 = reconstruction and Riemann flux of each direction in two
- *   kernels with the face states in HBM (default in 1D); 1 = one fused sweep kernel per
- *   direction, the face states kept on chip (default in 3D; 2nd and 4th-order interpolation,
- *   other orders keep the two kernels; at the 2nd order one launch for all directions).  The 2D
- *   default at the 4th order fuses x, and y for the HLLD solvers and on small grids.
+ *   kernels with the face states in HBM; 1 = one fused sweep kernel per direction, the face
+ *   states kept on chip (default in 3D; 2nd and 4th-order interpolation, other orders keep the
+ *   two kernels; at the 2nd order one launch for all directions).  The 2D default at the 4th
+ *   order fuses x, and y for the HLLD solvers and on small grids.  The 1D default is neither:
+ *   one kernel for a whole stage where it is built and faster (2nd and 4th order, RK2 and RK3,
+ *   up to a size by order and solver; not with the Hall or the Athena-type form), else 0; either
+ *   value switches that kernel off.
  *   QAS_OPT_LR_STAGING: 1 = the reconstruction stages its stencils in shared memory with
  *   TMA tensor copies (available for 2D/3D, 4th-order interpolation, even padded x extent;
  *   QAS_ERR_UNSUPPORTED otherwise); 0 = it reads them from global memory (default: measured
@@ -292,6 +297,8 @@ qas_status qas_set_gravity(qas_ctx *ctx, const double *phi_g);
 /* Failure-path hook: value != 0 makes the loop node of a captured dissipative step fail as on a driver without
  * conditional nodes, so that qas_run captures the guarded sub-cycles instead; 0 restores the default. */
 #define QAS_OPT_TEST_NO_LOOP 6
+/* qas_profile_run in 2D: 1 = the kernels that qas_run issues, 0 (default) = the face sweeps in two kernels. */
+#define QAS_OPT_PROFILE_AS_RUN 7
 qas_status qas_set_option(qas_ctx *ctx, int option, int value);
 
 /* Thread-block tile (tx*ty*tz <= 128 threads, tx a multiple of 32) of one cell kernel
@@ -302,6 +309,7 @@ qas_status qas_get_tile(const qas_ctx *ctx, const char *kernel, int *tx, int *ty
 /* Autotuner: for each cell kernel, time the candidate tiles over `trial_steps` exec_ steps
  * with CUDA events and keep the fastest.  The state, dt, time and step counter are restored
  * afterwards (results do not depend on the tile: every tile gives bit-identical states).
+ * Only kernels that a run of the context issues are timed; the tiles of the others stay.
  * Choices are cached per (dim, ODR, RMN, grid-size bucket) for the life of the process. */
 qas_status qas_autotune(qas_ctx *ctx, int trial_steps);
 
@@ -334,7 +342,8 @@ qas_status qas_batch_download(qas_batch *batch, int instance, double *block);
 /* exec_ loops of every instance; info (n entries, may be NULL) receives each instance's counters */
 qas_status qas_batch_run(qas_batch *batch, const qas_run_opts *opts, qas_run_info *info);
 qas_status qas_batch_set_tile(qas_batch *batch, const char *kernel, int tx, int ty, int tz);
-/* time candidate tiles per kernel over trial_steps steps (state restored) and keep the fastest */
+/* time candidate tiles per kernel over trial_steps steps (state restored) and keep the fastest; the steps are
+ * timed with the face sweeps in two kernels, the form of small ensembles and of orders without fused sweeps */
 qas_status qas_batch_autotune(qas_batch *batch, int trial_steps);
 qas_status qas_batch_stream(qas_batch *batch, void **stream);
 qas_status qas_batch_kernel_launches(const qas_batch *batch, long long *count);

@@ -190,6 +190,7 @@ struct qas_ctx {
   int sweep_seg[3] = {0, 0, 0};  // segment length of the fused y / z sweeps (0: not chosen yet)
   // live per-kernel timing (qas_profile_run): an event pair around every launch
   bool prof = false;
+  bool prof_as_run = false;  // QAS_OPT_PROFILE_AS_RUN
   std::vector<cudaEvent_t> prof_events;
   std::vector<int> prof_kids;  // kernel id of each recorded pair
   double prof_ms[32] = {0};
@@ -355,11 +356,11 @@ namespace {
 
 enum Kid {
   KID_PRIM, KID_DV, KID_LR, KID_FLUX, KID_EMF, KID_UPDATE, KID_BOUND, KID_BEGIN, KID_VMAX, KID_SETDT,
-  KID_ERES, KID_DFLUX, KID_DUPDATE, KID_DBOUND, KID_DCOPY, KID_DSUB, KID_SWEEP, KID_COUNT
+  KID_ERES, KID_DFLUX, KID_DUPDATE, KID_DBOUND, KID_DSUB, KID_SWEEP, KID_STAGE1, KID_COUNT
 };
 const char *const KID_NAMES[KID_COUNT] = {"k_prim", "k_dv", "k_lr", "k_flux", "k_emf", "k_update", "k_bound",
                                           "k_begin_step", "k_vmax", "k_setdt", "k_eres", "k_dflux",
-                                          "k_dupdate", "k_dbound", "k_dcopy", "k_dsub", "k_sweep"};
+                                          "k_dupdate", "k_dbound", "k_dsub", "k_sweep", "k_stage1"};
 
 void prof_mark(qas_ctx *c, int kid)
 {
@@ -772,8 +773,8 @@ long long stage_rest(qas_ctx *c, double c0, double c1)
 {
   const Geo &g = c->geo;
   long long nk = 0;
-  // a profile run keeps the 2D stage's two kernels apart, to time each
-  const bool split = !sweep_built(c) || (c->prof && g.dim == 2 && !c->fused_set);
+  // a profile run keeps the 2D stage's two kernels apart, to time each, unless the form was asked for
+  const bool split = !sweep_built(c) || (c->prof && g.dim == 2 && !c->fused_set && !c->prof_as_run);
   const unsigned axes = split ? 0u : c->fused & ((1u << g.dim) - 1u);
   auto two_kernels = [&](int a) {
     launch_lr<ODR>(c, a);
@@ -1093,7 +1094,7 @@ bool hall_active(const qas_ctx *c) { return c->hall && c->hall_di != 0; }
 bool ghosts_kept(const qas_ctx *c) { return !c->view.phi && !hall_active(c); }
 
 // 1D steps in one kernel a stage (qas_stage1d.cuh): the orders it is built for, at least two stages (a
-// block's neighbours read its cells while it writes), no Hall form, no form asked for or timed apart.
+// block's neighbours read its cells while it writes), no Hall form, no form asked for.
 // Brio-Wu 1024: 62.7 us a step in 17 launches, 22.6 us in 3.  On large grids launches no longer count, but the eight
 // cells in 64 that a block computes for its neighbours and the low occupancy do; one kernel / separate ones, us a
 // step: 4th order, 20 k cells HLLD 27 / 62, 262 k Roe 179 / 182, HLLD 159 / 167, LHLLD 167 / 175, MLAU 205 / 190, 400 k
@@ -1103,7 +1104,7 @@ bool one_kernel_stages(const qas_ctx *c)
 {
   const long long most = c->scheme.odr == 4 || c->scheme.rmn == 0 ? 1ll << 18 : c->scheme.rmn == 3 ? LLONG_MAX : 1ll << 21;
   return c->geo.dim == 1 && c->geo.nd <= most && (c->scheme.odr == 4 || c->scheme.odr == 2) && c->scheme.rk >= 2 &&
-         c->scheme.char_mode != 2 && !c->hall && !c->fused_set && !c->prof;
+         c->scheme.char_mode != 2 && !c->hall && !c->fused_set;
 }
 // everything that decides which kernels a step consists of and an option can change between two runs: a
 // graph captured in another form is not replayed (a one-kernel step leaves the ghosts to the run's end)
@@ -1127,13 +1128,13 @@ long long launch_step1(qas_ctx *c, int check_tim)
       v.uo[m] = rk == R - 1 ? b.u[m] : w[rk];
       v.u0[m] = b.u[m];
     }
-    launch(c, fn, nb, S1_NT, v, c0, c1, check_tim, rk == R - 1 ? 1 : 0);
+    QL(c, KID_STAGE1, launch(c, fn, nb, S1_NT, v, c0, c1, check_tim, rk == R - 1 ? 1 : 0));
   }
   return R;
 }
 
 // fill: the ghost fill at the start of the step
-long long launch_exec_step(qas_ctx *c, const qas_run_opts &o, int n_after, bool fill = true)
+long long launch_exec_step(qas_ctx *c, const qas_run_opts &o, int n_after, bool fill)
 {
   long long nk = 0;
   if (one_kernel_stages(c)) {
@@ -1818,11 +1819,17 @@ qas_status qas_profile_run(qas_ctx *c, const qas_run_opts *opts, int nsteps, qas
     c->prof_ms[k] = 0.0;
     c->prof_n[k] = 0;
   }
-  int n_host = c->h_ctl->n;
+  const int n0 = c->h_ctl->n;
+  int n_host = n0;
+  const bool fill = !ghosts_kept(c), one = one_kernel_stages(c);
+  if (!fill && !one) {  // as in qas_run
+    launch(c, k_bound<BOUND_START>, shell_grid(c->geo), BLK, c->view, 1);
+    c->launches++;
+  }
   c->prof = true;
   for (int st = 0; st < nsteps; st++) {
     c->prof_kids.clear();
-    c->launches += launch_exec_step(c, o, n_host + 1);
+    c->launches += launch_exec_step(c, o, n_host + 1, fill);
     n_host++;
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
@@ -1838,6 +1845,10 @@ qas_status qas_profile_run(qas_ctx *c, const qas_run_opts *opts, int nsteps, qas
   }
   c->prof = false;
   c->prof_kids.clear();
+  if (one) {
+    launch(c, k_bound_end, shell_grid(c->geo), BLK, c->view, n0);
+    c->launches++;
+  }
   if ((s = check_launch(c)) != QAS_OK) return s;
   int w = 0;
   for (int k = 0; k < KID_COUNT && w < max_entries; k++) {
@@ -2007,6 +2018,10 @@ qas_status qas_set_option(qas_ctx *c, int option, int value)
     c->sub_loop = true;
     return QAS_OK;
   }
+  if (option == QAS_OPT_PROFILE_AS_RUN) {
+    c->prof_as_run = value != 0;
+    return QAS_OK;
+  }
   if (option == QAS_OPT_PIPE_ITEMS) return pipe_set_items(c, value);
   if (option == QAS_OPT_PIPE_LANES) return pipe_set_lanes(c, value);
   return QAS_ERR_INVALID;
@@ -2129,7 +2144,11 @@ qas_status qas_autotune(qas_ctx *c, int trial_steps)
     c->h_ctl->done = 0;
     if ((s = write_ctl(c)) != QAS_OK) break;
     c->run_initialised = true;
-    if ((s = qas_profile_run(c, &o, trial_steps, kt, 32, &cnt)) != QAS_OK) break;
+    const bool keep = c->prof_as_run;
+    c->prof_as_run = true;  // tiles of the kernels that a run issues
+    s = qas_profile_run(c, &o, trial_steps, kt, 32, &cnt);
+    c->prof_as_run = keep;
+    if (s != QAS_OK) break;
     for (int e = 0; e < cnt; e++)
       for (int q = 0; q < 6; q++)
         if (!strcmp(kt[e].name, KID_NAMES[kids[q]]) && kt[e].total_ms < best_ms[q]) {

@@ -50,6 +50,7 @@ QAS_OPT_PIPE_ITEMS = 3
 QAS_OPT_PIPE_LANES = 4
 QAS_OPT_TEST_TMA_STALL = 5
 QAS_OPT_TEST_NO_LOOP = 6
+QAS_OPT_PROFILE_AS_RUN = 7
 
 
 class QasError(RuntimeError):

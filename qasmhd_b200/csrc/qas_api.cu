@@ -214,6 +214,15 @@ struct qas_ctx {
   PipeState *pipe = nullptr;  // qas_step_host: stage buffers, copy streams, item plan
 };
 
+// the kernels address an array by 32-bit byte offsets (at() in qas_kernels.cuh): less than 4 GB each.  A grid beyond
+// that would need 330 GB for its 77 arrays and is refused as one that no device holds
+static bool offsets_fit(const qas_grid &g)
+{
+  const double nx = (double)g.nxm + 2 * GH, ny = g.dim >= 2 ? (double)g.nym + 2 * GH : 1.0;
+  const double nz = g.dim >= 3 ? (double)g.nzm + 2 * GH : 1.0;
+  return nx * ny * nz * sizeof(double) < 4294967296.0;
+}
+
 // ---------------------------------------------------------------------------
 // ghost-fill maps: replay the reference's fill passes on (source, factor) pairs
 // ---------------------------------------------------------------------------
@@ -1222,6 +1231,7 @@ qas_status qas_create(qas_ctx **out, const qas_grid *grid, const qas_scheme *sch
   if (scheme->rmn < 0 || scheme->rmn > 3 || scheme->odr < 1 || scheme->odr > 4 || scheme->rk < 1 ||
       scheme->rk > 3 || scheme->char_mode < 0 || scheme->char_mode > 2)
     return QAS_ERR_INVALID;
+  if (!offsets_fit(gr)) return QAS_ERR_NOMEM;
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return QAS_ERR_NO_DEVICE;
   qas_ctx *c = new (std::nothrow) qas_ctx();

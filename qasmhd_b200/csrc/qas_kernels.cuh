@@ -126,8 +126,8 @@ __device__ __forceinline__ long long cidx(const Geo &g, int i, int j, int k)
   return (long long)g.nx * ((long long)g.ny * k + j) + i;
 }
 
-// element of an array by 32-bit byte offset (no array reaches 4 GB: the pool holds 77 of them): a base
-// from the kernel's parameters plus a 32-bit register needs no 64-bit address arithmetic
+// element of an array by 32-bit byte offset (offsets_fit: no array reaches 4 GB): a base from the kernel's
+// parameters plus a 32-bit register needs no 64-bit address arithmetic
 __device__ __forceinline__ const double *at(const double *p, unsigned o)
 {
   return reinterpret_cast<const double *>(reinterpret_cast<const char *>(p) + o);

@@ -43,24 +43,29 @@ ALG_BYTES_PER_CELL_UPDATE = 512  # 8 FP64 fields: stage 1 reads u^n, writes; sta
 #            fields, the centre and face normal fields and the shock detector (1 in 2D, 2 in 3D,
 #            MLAU/LHLLD); writes 7 fluxes and the central induction fluxes (1 in 2D, 2 in 3D):
 #            the face states never leave the SM
+#   k_stage1 (a 1D stage in one kernel) reads 8 fields, from the second stage on 7 of ut, and
+#            writes 7: 20 a stage on average
 KERNEL_ARRAYS = {
     "k_lr": {1: 8 + 14, 2: 9 + 16, 3: 9 + 18},
     "k_flux": {1: 15 + 8, 2: 14 + 1 + 2 + 2 + 8 + 1, 3: 14 + 1 + 4 + 3 + 8 + 2},
     "k_sweep": {1: 8 + 7, 2: 9 + 1 + 7 + 1, 3: 9 + 2 + 7 + 2},
+    "k_stage1": {1: 20},
 }
-# FP64 work per cell, counted by ncu (dadd + dmul + dfma instructions, and flops with a dfma
-# counted 2): k_lr on the 2D Orszag-Tang 1024^2 workload (ODR=4), k_sweep (MLAU) on KH 128^3
-# (1410-1432 per direction); profiles/shared_march_sweeps.md
-FP64_INSTR_PER_CELL = {"k_lr": 968.0, "k_sweep": 1424.0}
-FP64_FLOPS_PER_CELL = {"k_lr": 1304.0, "k_sweep": 1902.0}
-# ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch of the dominant kernel, per
-# workload: k_lr (y faces) of OT 1024^2; for KH 3D the KH 128^3 captures (136^3 padded cells: k_lr
-# x faces 200.12 + 314.29 MB; k_sweep the mean of its x, y, z launches, 376 + 369 + 366 MB / 3;
-# profiles/shared_march_sweeps.md) scaled by padded cells to 264^3 (traffic per cell is
-# size-independent: every array is streamed once, the 126 MB L2 holds no full array)
-KERNEL_TRAFFIC_PER_LAUNCH = {("k_lr", "ot2d_1024"): 78e6 + 115e6,
+# FP64 work per padded cell of one launch, counted by ncu (dadd + dmul + dfma instructions; flops with a
+# dfma counted 2): k_lr of OT 1024^2; k_sweep of OT 1024^2 (HLLD, mean of 1325 / 1353 along x / y) and of
+# KH 128^3 (MLAU, mean of 1445 / 1461 / 1463), whose figures KH 256^3 takes too.
+_KH = {"k_sweep": (1456.0, 1969.0)}
+FP64_PER_CELL = {"ot2d_1024": {"k_lr": (1002.0, 1373.0), "k_sweep": (1339.0, 1818.0)}, "kh3d_128": _KH, "kh3d_256": _KH}
+# ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch of the dominant kernel, per workload: k_lr
+# (y faces) and k_sweep (mean of 109 / 118 MB) of OT 1024^2; for KH 3D the KH 128^3 captures (136^3 padded
+# cells: k_lr x faces 200.12 + 314.29 MB; k_sweep the mean of 377 + 372 + 368 MB) scaled by padded cells to
+# 264^3 (traffic per cell is size-independent: every array is streamed once, the 126 MB L2 holds no full
+# array)
+KERNEL_TRAFFIC_PER_LAUNCH = {("k_lr", "ot2d_1024"): 78e6 + 112e6,
+                             ("k_sweep", "ot2d_1024"): (109e6 + 118e6) / 2,
                              ("k_lr", "kh3d_256"): (200.12e6 + 314.29e6) * (264 / 136) ** 3,
-                             ("k_sweep", "kh3d_256"): (376e6 + 369e6 + 366e6) / 3 * (264 / 136) ** 3}
+                             ("k_sweep", "kh3d_128"): (377e6 + 372e6 + 368e6) / 3,
+                             ("k_sweep", "kh3d_256"): (377e6 + 372e6 + 368e6) / 3 * (264 / 136) ** 3}
 
 
 def parse():
@@ -340,6 +345,7 @@ def second_workload(name, steps=20, warmup=3, windows=5, cpu_steps=3):
             b.synchronize()
             wins.append(a.elapsed_time(b) / steps)
         ms = statistics.median(wins)
+        ctx.set_option(L.QAS_OPT_PROFILE_AS_RUN, 1)
         prof = ctx.profile(min(steps, 10), flg=1, cfl=prob.cfl)
         host = torch.empty((8, prob.nd), dtype=torch.float64, pin_memory=True)
         ctx.download_into(host.numpy())
@@ -619,6 +625,7 @@ def main():
 
     # dominant kernel, timed live with CUDA events on the context's stream over
     # min(K, 10) eager steps after the timed region
+    ctx.set_option(L.QAS_OPT_PROFILE_AS_RUN, 1)
     prof = ctx.profile(min(args.steps, 10), flg=1, cfl=prob.cfl)
     dom = max(prof, key=lambda k: prof[k][1])
     dom_launches, dom_ms = prof[dom]
@@ -652,11 +659,12 @@ def main():
         "gpu_launches_basis": "kernel launches of one timed window of K steps",
         "clocks": clk,
     }
-    if dom in FP64_INSTR_PER_CELL:
+    if dom in FP64_PER_CELL.get(args.workload, {}):
         # the dominant kernel is FP64-bound: its FP64 rate against the measured DFMA peak
         fp64_peak = L.fp64_peak_tflops()
-        tflops = FP64_FLOPS_PER_CELL[dom] * prob.nd / (dom_ms_launch * 1e-3) / 1e12
-        pipe = FP64_INSTR_PER_CELL[dom] * prob.nd / (dom_ms_launch * 1e-3) / (fp64_peak * 1e12 / 2.0)
+        instr, flops = FP64_PER_CELL[args.workload][dom]
+        tflops = flops * prob.nd / (dom_ms_launch * 1e-3) / 1e12
+        pipe = instr * prob.nd / (dom_ms_launch * 1e-3) / (fp64_peak * 1e12 / 2.0)
         line["fp64"] = {"kernel": dom, "achieved_tflops": tflops, "peak_tflops": fp64_peak,
                         "frac": tflops / fp64_peak, "pipe_frac": pipe,
                         "basis": "ncu-counted FP64 flops per cell x cells / live launch time; peak = measured DFMA "

@@ -676,7 +676,9 @@ void sweep_prepare(qas_ctx *c)
 // the axes whose face states stay on chip by default (bit a).  3D: all.  2D: x, and y for the HLLD
 // solvers and on small grids, where a launch counts more than the march (OT / KH 1024^2, two kernels
 // against one, us: x HLLD 139 / 121, LHLLD 149 / 134, MLAU 152 / 139, Roe 162 / 162; y HLLD 138 / 136,
-// LHLLD 152 / 147, MLAU 147 / 157, Roe 161 / 178).  The line for y, KH, two kernels / fused, us a step of Roe and of
+// LHLLD 152 / 147, MLAU 147 / 157, Roe 161 / 178).  2nd order, one launch for all axes, KH 1024^2, two kernels / one
+// launch, us a step: Roe 1072 / 1097, HLLD 931 / 836, LHLLD 1035 / 951, MLAU 1041 / 1007; 500^2 Roe 287 / 286.  3D, KH 96^3: Roe
+// 2348 / 2064, HLLD 2040 / 1696, LHLLD 2237 / 1903, MLAU 2292 / 1957.  The line for y at the 4th order, KH, two kernels / fused, us a step of Roe and of
 // MLAU: 160^2 116 / 113, 125 / 122; 256^2 155 / 156, 160 / 161; 300^2 184 / 176, 187 / 186; 400^2 252 / 255, 249 / 250;
 // 450^2 305 / 306, 299 / 314; 100x2000 321 / 328, 315 / 333; 600^2 493 / 508, 472 / 488.  1D: none.
 unsigned fused_axes(const qas_ctx *c)
@@ -1709,8 +1711,7 @@ qas_status qas_dsptv(qas_ctx *c, double dt, double nu0, double eta0)
   const double idx = 1.0 / c->grid.dx, idy = 1.0 / c->grid.dy;
   const double idz = g.dim == 3 ? 1.0 / c->grid.dz : 0.0;
   launch(c, k_dsub_fixed, 1, 1, c->view, c->d_dctl, dt, idx, idy, idz);
-  // dsptv itself does not fill the ghosts first; launch_dsptv starts with a fill, so
-  // run the body without it: copy, stages
+  // one dsptv(dt) call: no fill before it, ut copied, the stages in place
   launch(c, k_dcopy, (unsigned)((g.nd + 255) / 256), 256, c->view, c->d_dctl, 0);
   long long nk = 2;
   for (int rk = 0; rk < c->scheme.rk; rk++) {

@@ -225,7 +225,7 @@ QAS_HD void wcns4_lr(const double f[5], double &fl, double &fr)
   fr = 0.125 * (+w2 * pr2 + w1 * pr1 + w0 * pr0);
 }
 
-// wcns4_lr with the same rounded results in fewer FP64 operations (115 -> 101 a field), the form the
+// wcns4_lr with the same rounded results in fewer FP64 operations (115 -> 106 a field), the form the
 // kernels run:
 //  * a product by a power of two feeding a sum is one FMA (p2fma);
 //  * the candidates carry the final factor 1/8 in their coefficients (3/8 f instead of 3 f, ...;

@@ -313,8 +313,8 @@ static __global__ void k_dv(View v)
 // ---------------------------------------------------------------------------
 // Bound by FP64 issue (2 cycles a warp instruction) and, at 22 warps per SM, by the latency of a
 // block's first loads.  Per launch, OT 1024^2 x / KH 128^3 z: 104 / 268 us with 1096 FP64 operations
-// a cell and one copy of the interpolation per field, 7 blocks (72 registers) 88 / 228 us with 972
-// operations and the pair loop of face_states_emit; 6 blocks 91 / 243, 8 blocks 92 / 237.
+// a cell and one copy of the interpolation per field, 7 blocks (72 registers) 88 / 228 us with 968
+// operations (1002 with today's reciprocal: OT 95 -> 95 us) and the pair loop of face_states_emit; 6 blocks 91 / 243, 8 blocks 92 / 237.
 #ifndef QAS_LR_MINB
 #define QAS_LR_MINB 7
 #endif
@@ -616,12 +616,12 @@ __global__ void __launch_bounds__(128, QAS_FLUX_MLAU_MINB) k_flux_mlau(View v)
 // by the latency of stencil loads.  Four warps on consecutive cells touch 8 planes a round where
 // four separate marches touch 20, so the planes stay in L1 (hit rate 28 -> 61 %); with slots instead of
 // registers, the pair loop and the prefetches, per launch at KH 128^3 (MLAU), x / y / z:
-// 388 / 435 / 427 -> 317 / 339 / 328 us.
+// 388 / 435 / 427 -> 317 / 339 / 328 us (on average 337 then, 347 with today's reciprocal and plain loads).
 // Resident-block caps per Riemann solver: 6 (80 registers; 7 blocks 332 / 341 / 333, 5 blocks
 // 345 / 370 / 355 us), Roe's 4 (its flux needs 128; 5 blocks are slower).  PR: 0 the characteristic or primitive reconstruction by
 // v.recon (the default scheme), -1 also the Athena-type form, whose code raises the kernels'
-// register pressure (spills 200 -> 820 B).  Built for 4th-order interpolation (the other orders
-// take the two-kernel form).
+// register pressure (spills 400-600 -> 1300-2000 B).  Built for the 4th order, and for the 2nd without the Athena-type
+// form (the others take the two kernels).
 // ---------------------------------------------------------------------------
 #ifndef QAS_SWEEP_MINB
 #define QAS_SWEEP_MINB 6
